@@ -233,23 +233,39 @@ __device__ __forceinline__ T weno_side(const T* w, T inv, bool plus,
   return plus ? weno_plus7<T, FAST>(w, inv) : weno_minus7<T, FAST>(w, inv);
 }
 
+// s > 0 ? max(minus, -plus, 0) : max(-minus, plus, 0), the Godunov upwind
+// value of one axis shared by the normal-speed and reinitialization terms
+// (lsm_level_set_evolution3d.f.in:209-231, lsm_reinitialization3d.f.in:
+// 158-199).  The reference squares max(phi^-, 0) and min(phi^+, 0)
+// separately; rounding is monotone, so the larger square is the square of the
+// larger value, and a zero's sign squares away.  The maxima keep the
+// reference's "a > b ? a : b" (MINUS_FIRST: a is the minus side), which
+// decides what a NaN side counts as.  In FP64 the sign of s goes into the
+// operands' sign bits and the comparison with 0 reads the high word (0 for a
+// negative number or a NaN), so that one comparison of the three runs on
+// the FP64 pipe, which bounds these kernels.  s = 0 or NaN: unused by the
+// callers.
+template <bool MINUS_FIRST>
+__device__ __forceinline__ float upwind_max0(float s, float plus, float minus) {
+  const float a = s > 0.0f ? -plus : plus, b = s > 0.0f ? minus : -minus;
+  return fmax2(MINUS_FIRST ? fmax2(b, a) : fmax2(a, b), 0.0f);
+}
+template <bool MINUS_FIRST>
+__device__ __forceinline__ double upwind_max0(double s, double plus, double minus) {
+  const int f = __double2hiint(s) & (int)0x80000000;
+  const double a = __hiloint2double(__double2hiint(plus) ^ f ^ (int)0x80000000,
+                                    __double2loint(plus));
+  const double b = __hiloint2double(__double2hiint(minus) ^ f, __double2loint(minus));
+  const double g = MINUS_FIRST ? fmax2(b, a) : fmax2(a, b);
+  return (unsigned)__double2hiint(g) <= 0x7ff00000u ? g : 0.0;
+}
+
 // Godunov |grad phi|^2 of the normal-speed term
-// (lsm_level_set_evolution3d.f.in:209-231): per axis, for vn > 0,
-// max(max(phi^-, 0)^2, min(phi^+, 0)^2).  Both operands are squares of
-// non-negative numbers (max(phi^-, 0) and -min(phi^+, 0)), and rounding is
-// monotone, so the larger square is the square of the larger of the two:
-// max(phi^-, -phi^+, 0)^2, the same value in two comparisons and one product
-// instead of three and two (a zero's sign, the only difference, squares away).
 template <typename T>
 __device__ __forceinline__ T godunov_sq2(T vn, T xp, T yp, T zp, T xm, T ym,
                                          T zm) {
-  const T z = T(0);
-  T ax, ay, az;
-  if (vn > z) {
-    ax = fmax2(fmax2(xm, -xp), z); ay = fmax2(fmax2(ym, -yp), z); az = fmax2(fmax2(zm, -zp), z);
-  } else {
-    ax = fmax2(fmax2(-xm, xp), z); ay = fmax2(fmax2(-ym, yp), z); az = fmax2(fmax2(-zm, zp), z);
-  }
+  const T ax = upwind_max0<true>(vn, xp, xm), ay = upwind_max0<true>(vn, yp, ym),
+          az = upwind_max0<true>(vn, zp, zm);
   T s = ax * ax;
   s = s + ay * ay;
   s = s + az * az;
@@ -266,13 +282,8 @@ __device__ __forceinline__ T reinit_cell(T pc, T xp, T yp, T zp, T xm, T ym,
                                          T zm, T dx_sq, bool use0,
                                          bool fp64_sign) {
   const T z = T(0);
-  T gp[3] = {xp, yp, zp}, gm[3] = {xm, ym, zm}, gs[3];
-  // per axis max(max(-+phi^+, 0), max(+-phi^-, 0)) as max(-+phi^+, +-phi^-, 0):
-  // the same value (but for a zero's sign, which squares away) in two
-  // comparisons instead of three
-#pragma unroll
-  for (int d = 0; d < 3; d++)
-    gs[d] = pc > z ? fmax2(fmax2(-gp[d], gm[d]), z) : fmax2(fmax2(gp[d], -gm[d]), z);
+  const T gs[3] = {upwind_max0<false>(pc, xp, xm), upwind_max0<false>(pc, yp, ym),
+                   upwind_max0<false>(pc, zp, zm)};
   // FP64 build's zero_tol for both precisions (see stage_zero_tol)
   if (!(fabsT(pc) >= T(1.0e-11))) return z;
   const T nsq = gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2];
@@ -701,9 +712,9 @@ template <> struct Pair2<float> { using type = float2; };
 // stage_tile_faces.
 constexpr int kPairPX = 4;
 
-template <typename T, bool K64, bool LMAX = false>
+template <typename T, bool K64>
 __device__ __forceinline__ void face_pm_t(const T* u, const FaceConst<T>& k, T& vp, T& vm) {
-  weno5_face<T, sizeof(T) == 4 && K64, LMAX>(u, k, vp, vm);
+  weno5_face<T, sizeof(T) == 4 && K64>(u, k, vp, vm);
 }
 
 template <typename T, int KIND, bool K64, int TX, int TY, int TZ>
@@ -874,11 +885,13 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
         weno5_face2(a, p.inv[2], vp, vm);
         zp0 = vp.x; zp1 = vp.y; znx0 = vm.x; znx1 = vm.y;
       } else {
-        face_pm_t<T, K64, true>(u, p.fk[0], xp0, xm1);   // shares its eps maximum's
-                                                          // inner part with the next
+        // the branches (the second cell's y and z faces) keep each block of
+        // straight-line code, and so the values live in it, small
+        face_pm_t<T, K64>(u, p.fk[0], xp0, xm1);
         face_pm_t<T, K64>(u + 1, p.fk[0], xp1, xnext);
         face_pm_t<T, K64>(ya, p.fk[1], yp0, ym0);
-        face_pm_t<T, K64>(yb, p.fk[1], yp1, ym1);
+        ym1 = T(0);
+        if (act1) face_pm_t<T, K64>(yb, p.fk[1], yp1, ym1);
         face_pm_t<T, K64>(w0 + 1, p.fk[2], zp0, znx0);
         if (act1) face_pm_t<T, K64>(w1 + 1, p.fk[2], zp1, znx1);
       }
@@ -896,17 +909,22 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
     if (act0) {
       const T2 ym = *reinterpret_cast<const T2*>(&fy[ty][c0]);
       const T xm0 = t == 0 ? fx[ty] : xm_left;
+      // both cells in one block of code: their chains of square roots overlap
+      // (a cell outside the fill box computes from zeros and stores nothing)
+      double h1 = -1.0;
       const T L0 =
           two_sided_rhs<T, KIND, true>(p, a00, w0[3], xp0, yp0, zp0, xm0, ym.x, zrun0, hmax);
+      const T L1 =
+          two_sided_rhs<T, KIND, true>(p, a01, w1[3], xp1, yp1, zp1, xm1, ym.y, zrun1, h1);
       zrun0 = znx0;
-      if (KIND == kStageNormalRhs) p.rhs_out[o0] = L0;
-      else p.out[o0] = stage_out(p, o0, uc0, w0[3], L0, dt);
+      zrun1 = znx1;
+      T* const dst = KIND == kStageNormalRhs ? p.rhs_out : p.out;
+      const T r0 = KIND == kStageNormalRhs ? L0 : stage_out(p, o0, uc0, w0[3], L0, dt);
+      const T r1 = KIND == kStageNormalRhs ? L1 : stage_out(p, o0 + 1, uc1, w1[3], L1, dt);
+      dst[o0] = r0;
       if (act1) {
-        const T L1 = two_sided_rhs<T, KIND, true>(p, a01, w1[3], xp1, yp1, zp1, xm1, ym.y,
-                                                  zrun1, hmax);
-        zrun1 = znx1;
-        if (KIND == kStageNormalRhs) p.rhs_out[o0 + 1] = L1;
-        else p.out[o0 + 1] = stage_out(p, o0 + 1, uc1, w1[3], L1, dt);
+        dst[o0 + 1] = r1;
+        if (KIND == kStageNormalRhs) hmax = h1 > hmax ? h1 : hmax;
       }
     }
   }

@@ -55,9 +55,12 @@ __device__ __forceinline__ float rsqrt_nr(float x) {
 }
 // sqrt(x) for x >= 0 as x / sqrt(x) with rsqrt_nr; x below the normal range
 // (where the ftz seed would be infinite) takes the correctly rounded sqrt
-template <typename T>
-__device__ __forceinline__ T sqrt_nr(T x) {
-  return x >= T(sizeof(T) == 8 ? 1e-300 : 1e-30) ? x * rsqrt_nr(x) : T(sqrt(x));
+// (in FP64 told by the high word: 2^-997 = 7e-301)
+__device__ __forceinline__ double sqrt_nr(double x) {
+  return __double2hiint(x) >= 0x01a00000 ? x * rsqrt_nr(x) : sqrt(x);
+}
+__device__ __forceinline__ float sqrt_nr(float x) {
+  return x >= 1e-30f ? x * rsqrt_nr(x) : sqrtf(x);
 }
 
 // a * b + c with one rounding, written out where an expression has two
@@ -83,6 +86,14 @@ __device__ __forceinline__ double inv_pow2_of(double x) {
 __device__ __forceinline__ float inv_pow2_of(float x) {
   const int e = (__float_as_int(x) >> 23) & 0xff;
   return __int_as_float((254 - e) << 23);
+}
+
+// x * inv_pow2_of(x), in [1, 2): the significand with the exponent of 1
+__device__ __forceinline__ double mantissa_of(double x) {
+  return __hiloint2double((__double2hiint(x) & 0xfffff) | 0x3ff00000, __double2loint(x));
+}
+__device__ __forceinline__ float mantissa_of(float x) {
+  return __int_as_float((__float_as_int(x) & 0x7fffff) | 0x3f800000);
 }
 
 // One side of HJ-WENO5 from the five undivided differences D1..D5 in the
@@ -208,11 +219,11 @@ static __device__ __noinline__ float2 weno5_face_fp64(float u0, float u1, float 
 // candidate scaled by it.
 template <typename T>
 struct FaceConst {
-  T inv, c3, c56, c16;   // 1/dx, 1/(3dx), 5/(6dx), 1/(6dx)
+  T inv, c2, c3, c16;   // 1/dx, 1/(2dx), 1/(3dx), 1/(6dx)
 };
 template <typename T>
 __host__ __device__ inline FaceConst<T> face_const(T inv) {
-  return {inv, inv * T(1.0 / 3.0), inv * T(5.0 / 6.0), inv * T(1.0 / 6.0)};
+  return {inv, inv * T(0.5), inv * T(1.0 / 3.0), inv * T(1.0 / 6.0)};
 }
 
 // The two HJ-WENO5 values that share the face between cells c and c+1, from
@@ -242,9 +253,7 @@ __host__ __device__ inline FaceConst<T> face_const(T inv) {
 //  * in FP64 one reciprocal of the product of the two weight sums serves
 //    both sides (the products stay below 2^230; in FP32 they would overflow,
 //    so FP32 takes two).
-// When KINK64 is set (FP32 form) a face whose indicators differ by more than
-// a factor 1e3 is recomputed in FP64.  Three further rearrangements, again
-// only rounding:
+// Three further rearrangements, again only rounding:
 //  * the S_k and eps enter the weights only through ratios of the q_k, so
 //    all four are taken four times over: S_k = 13/3 t1^2 + t2^2 (the
 //    reference's 13/12 t1^2 + 1/4 t2^2) and eps = 4e-6 max D^2 + 4 tiny;
@@ -253,29 +262,41 @@ __host__ __device__ inline FaceConst<T> face_const(T inv) {
 //    18 Pac shared;
 //  * 1/dx is folded into the middle candidate's weights (FaceConst) and
 //    into the one reciprocal.
-// LMAX: the eps maximum grouped as max(|D1|, max(|D2|..|D5|)) instead of
-// max(max(|D1|..|D4|), |D5|) -- the same value; a face evaluated with LMAX
-// beside the face one cell on (without) shares the inner four-way maximum.
-template <typename T, bool KINK64, bool LMAX = false>
+// From the second differences e_m = V_m+1 - V_m of u everything else is one
+// operation a value: ta = e2 - e1, tb = e3 - e2, tc = e4 - e3, the inner
+// terms of the indicators V1 - 4 V2 + 3 V3 = ta + 2 e2, V2 - V4 = -(e2 + e3),
+// 3 V3 - 4 V4 + V5 = tc - 2 e3, and the middle candidates p2m = V3 +
+// (2 e3 + e2)/6, p2p = p2m - (e2 + e3)/2.  A product 13/3 t^2 belongs to a
+// second difference of V, not to a face, so faces one cell apart share it
+// (with the e_m and t).  The factor 3 of both weight sums goes into the one
+// reciprocal.
+// 62 FP64 instructions a face (57 for the second of two faces one cell apart)
+// against 67 (61) with the indicators formed from V directly.  FP64 stages
+// at 256^3 (fill box), with the right-hand sides of upwind_max0 (stage.cuh):
+// reinitialization 403 -> 373 us, normal speed 414 -> 388 us.  Two faces
+// written in step, operation by operation, was slower (386 us: both faces'
+// values are live at once), as were eps maxima compared as 64-bit integers
+// (416 us: four integer instructions for one comparison).
+// When KINK64 is set (FP32 form) a face whose indicators differ by more than
+// a factor 1e3 is recomputed in FP64.
+template <typename T, bool KINK64>
 __device__ __forceinline__ void weno5_face(const T* u, const FaceConst<T>& k, T& vp, T& vm) {
   const T V1 = u[1] - u[0], V2 = u[2] - u[1], V3 = u[3] - u[2], V4 = u[4] - u[3],
           V5 = u[5] - u[4];
-  const T amax = LMAX ? vmax(fabs(V1), vmax(vmax(fabs(V2), fabs(V3)), vmax(fabs(V4), fabs(V5))))
-                      : vmax(vmax(vmax(fabs(V1), fabs(V2)), vmax(fabs(V3), fabs(V4))), fabs(V5));
+  const T amax =
+      vmax(vmax(vmax(fabs(V1), fabs(V2)), vmax(fabs(V3), fabs(V4))), fabs(V5));
   const T m = amax * amax;
   // four times the reference's 1e-6 max(v^2) + tiny, in units of the
   // undivided differences (the floor, reached only where every |D| < 1e-46,
   // is kept in these units)
   const T eps = fmaT(T(4e-6), m, T(4) * Consts<T>::tiny);
+  const T e1 = V2 - V1, e2 = V3 - V2, e3 = V4 - V3, e4 = V5 - V4;
+  const T ta = e2 - e1, tb = e3 - e2, tc = e4 - e3;
+  const T ra = fmaT(T(2), e2, ta), rb = e2 + e3, rc = fmaT(T(-2), e3, tc);
   const T c13_3 = T(13.0 / 3.0);
-  const T ta = fmaT(T(-2), V2, V1) + V3, tb = fmaT(T(-2), V3, V2) + V4,
-          tc = fmaT(T(-2), V4, V3) + V5;
-  T t = fmaT(T(3), V3, fmaT(T(-4), V2, V1));
-  const T Sa = fmaT(c13_3 * ta, ta, t * t);
-  t = V2 - V4;
-  const T Sb = fmaT(c13_3 * tb, tb, t * t);
-  t = fmaT(T(-4), V4, T(3) * V3) + V5;
-  const T Sc = fmaT(c13_3 * tc, tc, t * t);
+  const T Sa = fmaT(ra, ra, c13_3 * ta * ta);
+  const T Sb = fmaT(rb, rb, c13_3 * tb * tb);
+  const T Sc = fmaT(rc, rc, c13_3 * tc * tc);
   if (KINK64) {
     const T mx = vmax(vmax(Sa, Sb), Sc), mn = vmin(vmin(Sa, Sb), Sc);
     if (mx > T(1e3) * mn + T(4e-4) * m) {
@@ -287,27 +308,24 @@ __device__ __forceinline__ void weno5_face(const T* u, const FaceConst<T>& k, T&
       }
     }
   }
-  const T sc = inv_pow2_of(eps);
-  const T es = eps * sc;
+  const T sc = inv_pow2_of(eps), es = mantissa_of(eps);   // es = eps * sc
   const T qa = fmaT(Sa, sc, es), qb = fmaT(Sb, sc, es), qc = fmaT(Sc, sc, es);
   const T Qa = qa * qa, Qb = qb * qb, Qc = qc * qc;
   const T Pbc = Qb * Qc, Pac = Qa * Qc, Pab = Qa * Qb;
+  // 10 sm and 10 sp of the formulas above
+  const T sm = fmaT(T(3), Pab, fmaT(T(6), Pac, Pbc));
+  const T sp = fmaT(T(3), Pbc, fmaT(T(6), Pac, Pab));
   const T A = Pbc * (ta - tb), B = Pab * (tb - tc);
   const T num_m = fmaT(T(1.5), B, A), num_p = fmaT(T(1.5), A, B);
-  const T e3 = k.c56 * V3;
-  const T p2m = fmaT(k.c3, V4, fmaT(-k.c16, V2, e3));
-  const T p2p = fmaT(k.c3, V2, fmaT(-k.c16, V4, e3));
-  // 30 sm and 30 sp
-  const T p18 = T(18) * Pac;
-  const T sm = fmaT(T(3), Pbc, fmaT(T(9), Pab, p18));
-  const T sp = fmaT(T(3), Pab, fmaT(T(9), Pbc, p18));
+  const T p2m = fmaT(k.c3, e3, fmaT(k.c16, e2, k.inv * V3));
+  const T p2p = fmaT(-k.c2, rb, p2m);
   if constexpr (sizeof(T) == 8) {
-    const T r = rcp_nr(sm * sp) * k.inv;
+    const T r = rcp_nr(sm * sp) * k.c3;
     vm = fmaT(num_m, sp * r, p2m);
     vp = fmaT(-num_p, sm * r, p2p);
   } else {
-    vm = fmaT(num_m, rcp_nr(sm) * k.inv, p2m);
-    vp = fmaT(-num_p, rcp_nr(sp) * k.inv, p2p);
+    vm = fmaT(num_m, rcp_nr(sm) * k.c3, p2m);
+    vp = fmaT(-num_p, rcp_nr(sp) * k.c3, p2p);
   }
 }
 template <typename T, bool KINK64>
