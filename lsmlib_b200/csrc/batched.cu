@@ -82,18 +82,18 @@ __global__ void k_bump(unsigned* c) { *c += 1u; }
 #endif
 
 // one tile of the batch with a schedule's stage routine
-template <typename T, int TX, int TY, int TZ, int STAGING>
+template <typename T, int TX, int TY, int STAGING>
 __device__ __forceinline__ void batch_tile(const StageParams<T>& p, int bx, int by, int bz,
                                            int policy) {
   if constexpr (STAGING == kPairStaging) {
     __shared__ __align__(16) T tile[2][TY + 6][TX + 8];
     if (sizeof(T) == 4 && (policy & kFp64Kinks))
-      stage_tile_pairs_up<T, kStageAdvectConst, sizeof(T) == 4, TX, TY, TZ>(p, bx, by, bz, tile);
+      stage_tile_pairs_up<T, kStageAdvectConst, sizeof(T) == 4, TX, TY>(p, bx, by, bz, tile);
     else
-      stage_tile_pairs_up<T, kStageAdvectConst, false, TX, TY, TZ>(p, bx, by, bz, tile);
+      stage_tile_pairs_up<T, kStageAdvectConst, false, TX, TY>(p, bx, by, bz, tile);
   } else {
     __shared__ T tile[2][TY + 6][TX + 6];
-    stage_tile<T, kStageAdvectConst, true, TX, TY, TZ, STAGING>(p, bx, by, bz, tile);
+    stage_tile<T, kStageAdvectConst, true, TX, TY, STAGING>(p, bx, by, bz, tile);
   }
 }
 
@@ -137,7 +137,8 @@ k_batched_stage(const GridMeta* __restrict__ grids, const int4* __restrict__ ite
     p.use_phi0 = 0;
     p.fp64_policy = policy & kFp64Kinks;
     p.sr_seed = batch_sr_seed<T>(policy, sr_step, rk_kind);
-    batch_tile<T, TX, TY, TZ, STAGING>(p, it.y, it.z, it.w, policy);
+    p.tz = TZ;
+    batch_tile<T, TX, TY, STAGING>(p, it.y, it.z, it.w, policy);
   }
 }
 
@@ -224,7 +225,8 @@ k_grid_stage(const GridMeta* __restrict__ grids, int gi, T* out, const T* phi_s,
   p.use_phi0 = 0;
   p.fp64_policy = policy & kFp64Kinks;
   p.sr_seed = batch_sr_seed<T>(policy, sr_step, rk_kind);
-  batch_tile<T, TX, TY, TZ, STAGING>(p, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, policy);
+  p.tz = TZ;
+  batch_tile<T, TX, TY, STAGING>(p, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, policy);
 }
 
 std::mutex g_tune_mutex;

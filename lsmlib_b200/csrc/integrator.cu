@@ -357,7 +357,7 @@ bool band_setup(lsmgpu_workspace* ws, const void* phi, const FillBox& f, cudaStr
         !cuda_ok(cudaEventCreateWithFlags(&ws->band_ev[1], cudaEventDisableTiming), R))
       return false;
   }
-  const int tiles = stage_blocks(f);
+  const int tiles = stage_blocks(f, kStageTZ);
   if (ws->band_tiles < tiles) {
     if (ws->band_flags) cudaFree(ws->band_flags);
     ws->band_tiles = 0;
@@ -408,7 +408,7 @@ cudaError_t band_stage(int kind, lsmgpu_workspace* ws, const void* phi, StageArg
   b.fp64_policy = 0;
   b.sr_seed = 0u;
   if (!b.out || !b.phi_s || !b.phi_n) return cudaErrorInvalidValue;
-  return launch_stage_band(kind, a, b, ws->band_flags + stage_blocks(a.fb), st,
+  return launch_stage_band(kind, a, b, ws->band_flags + stage_blocks(a.fb, kStageTZ), st,
                            ws->band_stream, ws->band_ev);
 }
 
@@ -533,7 +533,9 @@ int lsmgpu_workspace_create(lsmgpu_workspace** out, const int gb[6],
   ws->npart = kAdvRedBlocks;
   FillBox whole;
   for (int d = 0; d < 3; d++) { whole.lo[d] = ws->gb.lo[d]; whole.hi[d] = ws->gb.hi(d); }
-  if (stage_blocks(whole) > ws->npart) ws->npart = stage_blocks(whole);
+  // every slab of a host-array call takes its own blocks
+  const int most = stage_blocks_max(whole) + kHostSlabs * kStageMaxSplit;
+  if (most > ws->npart) ws->npart = most;
   if (!(ws->phi1 = ws_alloc(ws->bytes, R)) || !(ws->phi2 = ws_alloc(ws->bytes, R)) ||
       !(ws->rhs = ws_alloc(ws->bytes, R)) ||
       !(ws->scal = (double*)ws_alloc(sizeof(double) * kNumScal, R)) ||
@@ -1057,7 +1059,6 @@ int lsmgpu_normal_tvdrk3_host(lsmgpu_workspace* ws, void* phi, const void* F,
   }
   if (!cuda_ok(cudaEventRecord(ws->up_ev[call % ws->nspeed], ci), R)) return LSMGPU_ERR_CUDA;
   const double tiny = ws->prec == 8 ? Consts<double>::tiny : (double)Consts<float>::tiny;
-  const int nblk = stage_blocks(f);
   void* dphi = ws->dphi;
   bool copied_back = false;
   for (int s = 0; s < nsteps; s++) {
@@ -1065,6 +1066,7 @@ int lsmgpu_normal_tvdrk3_host(lsmgpu_workspace* ws, void* phi, const void* F,
     a.aux[0] = dF;
     a.rhs_out = ws->rhs;
     a.phi_s = dphi;
+    int nblk = stage_blocks(f);
     if (s == 0) {
       // RHS/CFL pass of slab q once its planes and the 3 above have arrived
       int off = 0;
@@ -1077,6 +1079,7 @@ int lsmgpu_normal_tvdrk3_host(lsmgpu_workspace* ws, void* phi, const void* F,
         off += stage_blocks(b.fb);
         if (!cuda_ok(stage(kStageNormalRhs, ws->prec, b, st, ws), R)) return LSMGPU_ERR_CUDA;
       }
+      nblk = off;   // the slabs' own blocks
     } else {
       a.partials = ws->partials;
       if (!cuda_ok(stage(kStageNormalRhs, ws->prec, a, st, ws), R)) return LSMGPU_ERR_CUDA;

@@ -133,6 +133,7 @@ extern "C" int lsmgpu_normal_rhs_dt_noalloc(double* rhs, double* dt,
   a.aux[0] = F;
   a.rhs_out = rhs;
   a.partials = scratch;
+  a.tz = kStageTZ;   // the tiles counted above
   for (int d = 0; d < 3; d++) a.inv[d] = 1.0 / dx[d];
   double m = dx[0] > dx[1] ? dx[0] : dx[1];
   m = m > dx[2] ? m : dx[2];

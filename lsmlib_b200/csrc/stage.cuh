@@ -74,6 +74,7 @@ struct StageParams {
   const unsigned char* tile_fp64 = nullptr;
   unsigned tile_want = 0u;
   void* out_alt = nullptr;
+  int tz = 16;   // planes a block marches (stage_tz)
 };
 
 // LeVeque's 3D deformation velocity of a cell from its sine values and g,
@@ -336,7 +337,7 @@ __device__ __forceinline__ T weno_upwind_side(const T* w, T inv, bool plus,
 }
 
 // One tile of a fused stage: TX x TY cells (tile bx, by) marched over planes
-// [bz*TZ, bz*TZ + TZ) of the fill box.  ``tile`` holds two shared planes:
+// [bz*tz, bz*tz + tz) of the fill box (p.tz).  ``tile`` holds two shared planes:
 // plane k is written into buffer (k-kb)&1 while the other buffer may still be
 // read by slower threads of the previous plane.  Returns the tile's largest
 // CFL speed for kStageNormalRhs (-1 otherwise).  The caller synchronises the
@@ -346,15 +347,15 @@ __device__ __forceinline__ T weno_upwind_side(const T* w, T inv, bool plus,
 // plane); 1 reads the x and y neighbours straight from global memory through
 // L1 (no shared plane, no barrier; neighbouring threads share the cache
 // lines).  The batched autotuner picks one per batch.
-template <typename T, int KIND, bool FAST, int TX, int TY, int TZ, int STAGING = 0>
+template <typename T, int KIND, bool FAST, int TX, int TY, int STAGING = 0>
 __device__ __forceinline__ double stage_tile(const StageParams<T>& p, int bx,
                                              int by, int bz,
                                              T (*tile)[TY + 6][TX + 6]) {
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i = p.fb.lo[0] + bx * TX + tx;
   const int j = p.fb.lo[1] + by * TY + ty;
-  const int kb = p.fb.lo[2] + bz * TZ;
-  const int ke = min(kb + TZ - 1, p.fb.hi[2]);
+  const int kb = p.fb.lo[2] + bz * p.tz;
+  const int ke = min(kb + p.tz - 1, p.fb.hi[2]);
   const bool act = (i <= p.fb.hi[0]) && (j <= p.fb.hi[1]);
   const Grid3<const T> phi = make_grid(p.phi_s, p.gb);
   const long sy = p.gb.sy(), sz = p.gb.sz();
@@ -566,7 +567,7 @@ __device__ __forceinline__ void face_pm(const T* u, T inv, bool kink64, T& vp,
 // and z run are evaluated once more (rows by warp 0, columns by the last
 // warp, z at the first plane).  Tile staging, boundary values and prefetch
 // are those of stage_tile.
-template <typename T, int KIND, int TX, int TY, int TZ>
+template <typename T, int KIND, int TX, int TY>
 __device__ __forceinline__ double stage_tile_faces(const StageParams<T>& p, int bx,
                                                    int by, int bz,
                                                    T (*tile)[TY + 6][TX + 6],
@@ -576,8 +577,8 @@ __device__ __forceinline__ double stage_tile_faces(const StageParams<T>& p, int 
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i = p.fb.lo[0] + bx * TX + tx;
   const int j = p.fb.lo[1] + by * TY + ty;
-  const int kb = p.fb.lo[2] + bz * TZ;
-  const int ke = min(kb + TZ - 1, p.fb.hi[2]);
+  const int kb = p.fb.lo[2] + bz * p.tz;
+  const int ke = min(kb + p.tz - 1, p.fb.hi[2]);
   const bool act = (i <= p.fb.hi[0]) && (j <= p.fb.hi[1]);
   const Grid3<const T> phi = make_grid(p.phi_s, p.gb);
   const long sy = p.gb.sy(), sz = p.gb.sz();
@@ -712,28 +713,41 @@ template <> struct Pair2<float> { using type = float2; };
 // stage_tile_faces.
 constexpr int kPairPX = 4;
 
+// A block of kPairThreads threads covers kPairTX x kPairTY cells of a plane
+// as rows of 16 pairs.  The last column of tiles is narrower where the fill
+// box is not a multiple of kPairTX wide; with 16 or fewer columns left the
+// same threads take rows of 8 pairs (16 x 16 cells) or 4 (8 x 32 cells), so
+// that the column needs a half or a quarter of the blocks (the others
+// return at once).  A grid of 2^m cells has 2^m + 1 points along each axis:
+// one column in 33 (9 at 256) would otherwise run with 1 of its 32 columns.
+constexpr int kPairTX = 32, kPairTY = 8, kPairThreads = 128;
+constexpr int kPairRows = kPairThreads / 4 + 6;   // rows of the tallest tile and its halo
+__device__ __forceinline__ int pair_row_bits(int columns_left) {
+  return columns_left <= 8 ? 2 : columns_left <= 16 ? 3 : 4;
+}
+
 template <typename T, bool K64>
 __device__ __forceinline__ void face_pm_t(const T* u, const FaceConst<T>& k, T& vp, T& vm) {
   weno5_face<T, sizeof(T) == 4 && K64>(u, k, vp, vm);
 }
 
-template <typename T, int KIND, bool K64, int TX, int TY, int TZ>
+template <typename T, int KIND, bool K64>
 __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int bx, int by,
-                                                   int bz, T (*tile)[TY + 6][TX + 8],
-                                                   T (*fy)[TX], T* fx) {
+                                                   int bz, T (*tile)[kPairRows][kPairTX + 8],
+                                                   T* fy, T* fx) {
   using T2 = typename Pair2<T>::type;
-  static_assert(TX == 32, "a tile row is one half-warp of pairs");
-  static_assert(TY <= TX / 2, "row-start faces are spread over one row of threads");
-  static_assert(TY >= 3, "row 0 and the last two rows are distinct");
-  constexpr int NP = TX / 2;   // threads per row
   constexpr int PX = kPairPX;
-  const int t = threadIdx.x, ty = threadIdx.y;
-  const int x0 = p.fb.lo[0] + bx * TX, j0 = p.fb.lo[1] + by * TY;
+  const int x0 = p.fb.lo[0] + bx * kPairTX;
+  const int lp = pair_row_bits(p.fb.hi[0] - x0 + 1);
+  const int NP = 1 << lp, TX = 2 * NP, TY = kPairThreads >> lp;
+  const int tid = threadIdx.x, t = tid & (NP - 1), ty = tid >> lp;
+  const int j0 = p.fb.lo[1] + by * TY;
+  if (j0 > p.fb.hi[1]) return -1.0;   // a narrow column has fewer tiles
   const int c0 = 2 * t;
   const int i0 = x0 + c0, i1 = i0 + 1;
   const int j = j0 + ty;
-  const int kb = p.fb.lo[2] + bz * TZ;
-  const int ke = min(kb + TZ - 1, p.fb.hi[2]);
+  const int kb = p.fb.lo[2] + bz * p.tz;
+  const int ke = min(kb + p.tz - 1, p.fb.hi[2]);
   const int hi0 = p.fb.hi[0], hi1 = p.fb.hi[1];
   const bool rowin = j <= hi1;
   const bool act0 = rowin && i0 <= hi0, act1 = rowin && i1 <= hi0;
@@ -765,16 +779,16 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
   const bool has_hy = (ty < 3) || (ty >= TY - 3 && rowin);
   const bool hy0 = has_hy && i0 <= hi0, hy1 = has_hy && i1 <= hi0;
   const int trow = ty < 3 ? ty : ty + 6;
-  // faces in front of rows (row 0, thread t < TY serves row t) and columns
+  // faces in front of rows (thread tid < TY serves row tid) and columns
   // (rows TY-2 and TY-1: column 2t and 2t+1 respectively)
-  const bool row_start = ty == 0 && t < TY && j0 + t <= hi1;
+  const bool row_start = tid < TY && j0 + tid <= hi1;
   const int col_c = c0 + (ty == TY - 1 ? 1 : 0);
   const bool col_start = ty >= TY - 2 && x0 + col_c <= hi0;
   // the extra face as a strided read of buffer 0 (buffer 1 is one tile on)
   const bool xtra = row_start || col_start;
-  const int xoff = row_start ? (t + 3) * (TX + 8) + PX - 3 : col_c + PX;
-  const int xstride = row_start ? 1 : TX + 8;
-  T* const xout = row_start ? &fx[t] : &fy[0][col_c];
+  const int xoff = row_start ? (tid + 3) * (kPairTX + 8) + PX - 3 : col_c + PX;
+  const int xstride = row_start ? 1 : kPairTX + 8;
+  T* const xout = row_start ? &fx[tid] : &fy[col_c];
 
   // 32-bit element offsets from the index-space origin (the launcher takes
   // this kernel only for arrays of fewer than 2^31 elements): the 64-bit
@@ -895,7 +909,7 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
         face_pm_t<T, K64>(w0 + 1, p.fk[2], zp0, znx0);
         if (act1) face_pm_t<T, K64>(w1 + 1, p.fk[2], zp1, znx1);
       }
-      if (ty + 1 < TY) *reinterpret_cast<T2*>(&fy[ty + 1][c0]) = T2{ym0, ym1};
+      if (ty + 1 < TY) *reinterpret_cast<T2*>(&fy[2 * tid + TX]) = T2{ym0, ym1};
     }
     const T xm_left = __shfl_up_sync(0xffffffffu, xnext, 1, NP);
     if (xtra) {
@@ -907,7 +921,7 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
     }
     __syncthreads();
     if (act0) {
-      const T2 ym = *reinterpret_cast<const T2*>(&fy[ty][c0]);
+      const T2 ym = *reinterpret_cast<const T2*>(&fy[2 * tid]);   // row ty, column c0
       const T xm0 = t == 0 ? fx[ty] : xm_left;
       // both cells in one block of code: their chains of square roots overlap
       // (a cell outside the fill box computes from zeros and stores nothing)
@@ -945,23 +959,32 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
 // of stage_tile (weno_upwind_side and the same RHS and RK update), but for
 // FP32 without the FP64 kink recomputation, where the two cells' sides of
 // an axis are one packed FP32x2 evaluation (weno5_side2).
-// BAND: the FP64 band form (out_alt written as well).
-template <typename T, int KIND, bool K64, int TX, int TY, int TZ, bool BAND = false>
-__device__ __forceinline__ void stage_tile_pairs_up(const StageParams<T>& p, int bx, int by,
-                                                    int bz, T (*tile)[TY + 6][TX + 8]) {
+// BAND: the FP64 band form (out_alt written as well).  NARROW: the last
+// column of tiles may take shorter rows (pair_row_bits), block of
+// kPairThreads threads.
+template <typename T, int KIND, bool K64, int TX_, int TY_, bool BAND = false, bool NARROW = false>
+__device__ __forceinline__ void stage_tile_pairs_up(
+    const StageParams<T>& p, int bx, int by, int bz,
+    T (*tile)[NARROW ? kPairRows : TY_ + 6][TX_ + 8]) {
   using T2 = typename Pair2<T>::type;
   // (no lane exchange: a row of TX/2 >= 4 threads of any width works)
-  static_assert(TX % 2 == 0 && TX / 2 >= 4, "strip roles need four threads per row");
-  static_assert(TY >= 3, "the y strips need three rows at each end");
-  constexpr int NP = TX / 2;
+  static_assert(TX_ % 2 == 0 && TX_ / 2 >= 4, "strip roles need four threads per row");
+  static_assert(TY_ >= 3, "the y strips need three rows at each end");
+  static_assert(!NARROW || (TX_ == kPairTX && TY_ == kPairTY), "narrow columns: 32 x 8 tiles");
   constexpr int PX = kPairPX;
-  const int t = threadIdx.x, ty = threadIdx.y;
-  const int x0 = p.fb.lo[0] + bx * TX, j0 = p.fb.lo[1] + by * TY;
+  const int x0 = p.fb.lo[0] + bx * TX_;
+  const int lp = NARROW ? pair_row_bits(p.fb.hi[0] - x0 + 1) : 0;
+  const int NP = NARROW ? 1 << lp : TX_ / 2;
+  const int TX = 2 * NP, TY = NARROW ? kPairThreads >> lp : TY_;
+  const int t = NARROW ? threadIdx.x & (NP - 1) : threadIdx.x;
+  const int ty = NARROW ? threadIdx.x >> lp : threadIdx.y;
+  const int j0 = p.fb.lo[1] + by * TY;
+  if (NARROW && j0 > p.fb.hi[1]) return;   // a narrow column has fewer tiles
   const int c0 = 2 * t;
   const int i0 = x0 + c0, i1 = i0 + 1;
   const int j = j0 + ty;
-  const int kb = p.fb.lo[2] + bz * TZ;
-  const int ke = min(kb + TZ - 1, p.fb.hi[2]);
+  const int kb = p.fb.lo[2] + bz * p.tz;
+  const int ke = min(kb + p.tz - 1, p.fb.hi[2]);
   const int hi0 = p.fb.hi[0], hi1 = p.fb.hi[1];
   const bool rowin = j <= hi1;
   const bool act0 = rowin && i0 <= hi0, act1 = rowin && i1 <= hi0;
@@ -1167,7 +1190,7 @@ __device__ __forceinline__ void block_max_partial(const P& p, double hmax) {
 #define LSMGPU_STAGE_MIN_BLOCKS (768 / (TX * TY))
 #endif
 
-template <typename T, int KIND, bool FAST, int TX, int TY, int TZ>
+template <typename T, int KIND, bool FAST, int TX, int TY>
 __global__ void __launch_bounds__(TX * TY, LSMGPU_STAGE_MIN_BLOCKS)
 k_stage(StageParams<T> p) {
   __shared__ T tile[2][TY + 6][TX + 6];
@@ -1175,10 +1198,10 @@ k_stage(StageParams<T> p) {
   if constexpr (UseFaces<T, KIND, FAST, TX>::value) {
     __shared__ T fy[TY][TX];
     __shared__ T fx[TY];
-    hmax = stage_tile_faces<T, KIND, TX, TY, TZ>(p, (int)blockIdx.x, (int)blockIdx.y,
+    hmax = stage_tile_faces<T, KIND, TX, TY>(p, (int)blockIdx.x, (int)blockIdx.y,
                                                  (int)blockIdx.z, tile, fy, fx);
   } else {
-    hmax = stage_tile<T, KIND, FAST, TX, TY, TZ>(p, (int)blockIdx.x, (int)blockIdx.y,
+    hmax = stage_tile<T, KIND, FAST, TX, TY>(p, (int)blockIdx.x, (int)blockIdx.y,
                                                  (int)blockIdx.z, tile);
   }
   block_max_partial<KIND, TX * TY>(p, hmax);
@@ -1190,33 +1213,34 @@ k_stage(StageParams<T> p) {
 #endif
 
 // The face-shared two-sided kinds, two cells per thread (stage_tile_pairs):
-// a block of TX/2 x TY threads covers the same TX x TY x TZ tile as k_stage.
+// a block of kPairThreads threads covers the same 32 x 8 x tz tile as k_stage.
 // Every ghost cell the stencils reach is read as stored.
-template <typename T, int KIND, bool K64, int TX, int TY, int TZ>
-__global__ void __launch_bounds__(TX / 2 * TY, LSMGPU_PAIR_MIN_BLOCKS)
+template <typename T, int KIND, bool K64>
+__global__ void __launch_bounds__(kPairThreads, LSMGPU_PAIR_MIN_BLOCKS)
 k_stage_pairs(StageParams<T> p) {
-  __shared__ __align__(16) T tile[2][TY + 6][TX + 8];
-  __shared__ __align__(16) T fy[TY][TX];
-  __shared__ T fx[TY];
-  const double hmax = stage_tile_pairs<T, KIND, K64, TX, TY, TZ>(
-      p, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, tile, fy, fx);
-  block_max_partial<KIND, TX / 2 * TY>(p, hmax);
+  __shared__ __align__(16) T tile[2][kPairRows][kPairTX + 8];
+  __shared__ __align__(16) T fy[2 * kPairThreads + kPairTX];
+  __shared__ T fx[kPairThreads / 4];
+  const double hmax = stage_tile_pairs<T, KIND, K64>(p, (int)blockIdx.x, (int)blockIdx.y,
+                                                     (int)blockIdx.z, tile, fy, fx);
+  block_max_partial<KIND, kPairThreads>(p, hmax);
 }
 
 // The one-sided kinds, two cells per thread (stage_tile_pairs_up); every
 // ghost cell the stencils reach is read as stored.  BAND: the FP64 band form
-// (the tiles whose tile_fp64 flag is tile_want, out_alt written as well).
-template <typename T, int KIND, bool K64, int TX, int TY, int TZ, bool BAND = false>
-__global__ void __launch_bounds__(TX / 2 * TY, LSMGPU_PAIR_MIN_BLOCKS)
+// (the tiles whose tile_fp64 flag is tile_want, out_alt written as well; the
+// flags number 32 x 8 x kStageTZ tiles, so its columns are never narrow).
+template <typename T, int KIND, bool K64, bool BAND = false>
+__global__ void __launch_bounds__(kPairThreads, LSMGPU_PAIR_MIN_BLOCKS)
 k_stage_pairs_up(StageParams<T> p) {
-  __shared__ __align__(16) T tile[2][TY + 6][TX + 8];
+  __shared__ __align__(16) T tile[2][BAND ? kPairTY + 6 : kPairRows][kPairTX + 8];
   if constexpr (BAND) {
     if (p.tile_fp64[blockIdx.x + gridDim.x * (blockIdx.y + (size_t)gridDim.y * blockIdx.z)] !=
         p.tile_want)
       return;
   }
-  stage_tile_pairs_up<T, KIND, K64, TX, TY, TZ, BAND>(p, (int)blockIdx.x, (int)blockIdx.y,
-                                                     (int)blockIdx.z, tile);
+  stage_tile_pairs_up<T, KIND, K64, kPairTX, kPairTY, BAND, !BAND>(
+      p, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, tile);
 }
 
 // The face ghost cells of phi that the stencils of fill-box cells in planes

@@ -39,6 +39,7 @@ StageParams<T> to_params(const StageArgs& a) {
   p.defo_tab = a.defo_tab;
   for (int d = 0; d < 3; d++) p.defo_off[d] = a.defo_off[d];
   p.g_dev = a.g_dev;
+  p.tz = a.tz ? a.tz : stage_tz(a.fb);
   return p;
 }
 
@@ -89,7 +90,8 @@ bool pairs_apply(const StageArgs& a) {
 // the same.
 template <typename T, int KIND>
 void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStream_t st) {
-  constexpr int TX = kStageTX, TY = kStageTY, TZ = kStageTZ;
+  constexpr int TX = kStageTX, TY = kStageTY;
+  static_assert(TX == kPairTX && TY == kPairTY, "one tiling for all stage kernels");
   if constexpr (LSMGPU_STAGE_PAIRS && UseFaces<T, KIND, STAGE_FAST, TX>::value) {
     if (pairs_apply(a)) {
       StageParams<T> q = p;
@@ -97,14 +99,13 @@ void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStr
         launch_face_ghosts<T>(a, st);
         q.bc_mask = 0u;
       }
-      const dim3 blk(TX / 2, TY, 1);
       if constexpr (sizeof(T) == 4) {
         if (p.fp64_policy & kFp64Kinks) {
-          k_stage_pairs<T, KIND, true, TX, TY, TZ><<<grid, blk, 0, st>>>(q);
+          k_stage_pairs<T, KIND, true><<<grid, kPairThreads, 0, st>>>(q);
           return;
         }
       }
-      k_stage_pairs<T, KIND, false, TX, TY, TZ><<<grid, blk, 0, st>>>(q);
+      k_stage_pairs<T, KIND, false><<<grid, kPairThreads, 0, st>>>(q);
       return;
     }
   }
@@ -115,27 +116,26 @@ void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStr
         launch_face_ghosts<T>(a, st);
         q.bc_mask = 0u;
       }
-      const dim3 blk(TX / 2, TY, 1);
       if constexpr (sizeof(T) == 4) {
         if (p.fp64_policy & kFp64Kinks) {
-          k_stage_pairs_up<T, KIND, true, TX, TY, TZ><<<grid, blk, 0, st>>>(q);
+          k_stage_pairs_up<T, KIND, true><<<grid, kPairThreads, 0, st>>>(q);
           return;
         }
       }
-      k_stage_pairs_up<T, KIND, false, TX, TY, TZ><<<grid, blk, 0, st>>>(q);
+      k_stage_pairs_up<T, KIND, false><<<grid, kPairThreads, 0, st>>>(q);
       return;
     }
   }
-  k_stage<T, KIND, STAGE_FAST, TX, TY, TZ><<<grid, dim3(TX, TY, 1), 0, st>>>(p);
+  k_stage<T, KIND, STAGE_FAST, TX, TY><<<grid, dim3(TX, TY, 1), 0, st>>>(p);
 }
 
 template <typename T>
 cudaError_t launch_t(int kind, const StageArgs& a, cudaStream_t st) {
-  constexpr int TX = kStageTX, TY = kStageTY, TZ = kStageTZ;
+  constexpr int TX = kStageTX, TY = kStageTY;
   const FillBox& fb = a.fb;
-  dim3 grid((fb.n(0) + TX - 1) / TX, (fb.n(1) + TY - 1) / TY,
-            (fb.n(2) + TZ - 1) / TZ);
   const StageParams<T> p = to_params<T>(a);
+  const dim3 grid((fb.n(0) + TX - 1) / TX, (fb.n(1) + TY - 1) / TY,
+                  (fb.n(2) + p.tz - 1) / p.tz);
   switch (kind) {
     case kStageAdvect: launch_kind<T, kStageAdvect>(grid, a, p, st); break;
     case kStageNormal: launch_kind<T, kStageNormal>(grid, a, p, st); break;
@@ -156,7 +156,7 @@ template <int KIND>
 cudaError_t band_kind(dim3 grid, const StageArgs& a32, const StageArgs& a64,
                       const unsigned char* tile_fp64, cudaStream_t st, cudaStream_t side,
                       cudaEvent_t ev[2]) {
-  constexpr int TX = kStageTX, TY = kStageTY, TZ = kStageTZ;
+  constexpr int TX = kStageTX, TY = kStageTY;
   static_assert(UsePairsUp<float, KIND, STAGE_FAST, TX>::value &&
                     UsePairsUp<double, KIND, STAGE_FAST, TX>::value,
                 "the band form runs the two-cells-per-thread upwind kernels");
@@ -171,6 +171,7 @@ cudaError_t band_kind(dim3 grid, const StageArgs& a32, const StageArgs& a64,
   q32.tile_fp64 = q64.tile_fp64 = tile_fp64;
   q32.tile_want = 0u;
   q64.tile_want = 1u;
+  q32.tz = q64.tz = kStageTZ;   // the tiles that the flags number
   q32.out_alt = a64.out;
   q64.out_alt = a32.out;
   const dim3 blk(TX / 2, TY, 1);
@@ -178,11 +179,11 @@ cudaError_t band_kind(dim3 grid, const StageArgs& a32, const StageArgs& a64,
   if ((e = cudaEventRecord(ev[0], st)) != cudaSuccess ||
       (e = cudaStreamWaitEvent(side, ev[0], 0)) != cudaSuccess)
     return e;
-  k_stage_pairs_up<double, KIND, false, TX, TY, TZ, true><<<grid, blk, 0, side>>>(q64);
+  k_stage_pairs_up<double, KIND, false, true><<<grid, blk, 0, side>>>(q64);
   if (q32.fp64_policy & kFp64Kinks)
-    k_stage_pairs_up<float, KIND, true, TX, TY, TZ, true><<<grid, blk, 0, st>>>(q32);
+    k_stage_pairs_up<float, KIND, true, true><<<grid, blk, 0, st>>>(q32);
   else
-    k_stage_pairs_up<float, KIND, false, TX, TY, TZ, true><<<grid, blk, 0, st>>>(q32);
+    k_stage_pairs_up<float, KIND, false, true><<<grid, blk, 0, st>>>(q32);
   launch_counter() += 2;
   if ((e = cudaEventRecord(ev[1], side)) != cudaSuccess ||
       (e = cudaStreamWaitEvent(st, ev[1], 0)) != cudaSuccess)

@@ -32,23 +32,59 @@ struct StageArgs {
   // arrays these are): the face-shared kinds then store the boundary values
   // of bc_mask into phi_s's ghost cells and read them as stored
   int ghosts_writable;
+  int tz;  // planes per block (0: stage_tz of the fill box)
 };
 
-// tile of the stage kernels: TX x TY cells per block, TZ planes per block
-// (build-time settings; TX is one warp)
-#ifndef LSMGPU_STAGE_TY
-#define LSMGPU_STAGE_TY 8
-#endif
-#ifndef LSMGPU_STAGE_TZ
-#define LSMGPU_STAGE_TZ 16
-#endif
-constexpr int kStageTX = 32, kStageTY = LSMGPU_STAGE_TY, kStageTZ = LSMGPU_STAGE_TZ;
+// Tile of the stage kernels: TX x TY cells of a plane, marched over stage_tz
+// planes (kStageTZ in the FP64 band form, whose flags number the tiles).
+constexpr int kStageTX = 32, kStageTY = 8, kStageTZ = 16;
+constexpr int kStageMaxTZ = 11;         // the longest march otherwise
+constexpr int kStageMaxSplit = 4096;    // shorter marches: at most this many blocks
 
-inline int stage_blocks(const FillBox& fb) {
+inline int stage_blocks(const FillBox& fb, int tz) {
   const int gx = (fb.n(0) + kStageTX - 1) / kStageTX;
   const int gy = (fb.n(1) + kStageTY - 1) / kStageTY;
-  const int gz = (fb.n(2) + kStageTZ - 1) / kStageTZ;
+  const int gz = (fb.n(2) + tz - 1) / tz;
   return gx * gy * gz;
+}
+
+// Planes a block marches: the tz of the smallest estimated time.  A block
+// takes about tz + 2 planes (the window loads and the extra z faces cost
+// two), and a plane 2.1, 2.6, 3.2 or 3.5 us with 1 to 4 blocks on its SM
+// (more do not fit); blocks that follow one another without a common start
+// take 2.75 (measured on the FP64 reinitialization stage; the ratios hold for
+// the other kinds and FP32).  Small grids so get thin slabs that reach every
+// SM, larger ones slabs that end together: with 16 planes for every grid the
+// stage took 41.0 us at 33^3 (30 blocks), 43.0 at 65^3, 66.2 at
+// 130x98x132, now 12.4, 20.5 and 58.  Past 11 planes nothing is gained: 16
+// against 11 at 257^3 measured 407 and 404 us (reinitialization), 464 and 446
+// (velocity arrays).
+inline int stage_tz(const FillBox& fb) {
+  constexpr int kSms = 148, kSlots = 4 * kSms;
+  constexpr double kSteady = 2.75, kPlane[5] = {0.0, 2.1, 2.6, 3.2, 3.5};
+  const int left = fb.n(0) % kStageTX;   // the last column's width (pair_row_bits)
+  const int ly = left <= 8 ? 4 * kStageTY : left <= 16 ? 2 * kStageTY : kStageTY;
+  const long tiles = (long)(fb.n(0) / kStageTX) * ((fb.n(1) + kStageTY - 1) / kStageTY) +
+                     (left ? (fb.n(1) + ly - 1) / ly : 0);
+  int best = kStageMaxTZ;
+  double best_cost = 0.0;
+  for (int tz = kStageMaxTZ; tz >= 1; tz--) {
+    if (stage_blocks(fb, tz) > kStageMaxSplit) break;
+    const long blocks = tiles * ((fb.n(2) + tz - 1) / tz);
+    const double cost = (tz + 2) * ((double)(blocks / kSlots) * kSteady +
+                                    kPlane[(blocks % kSlots + kSms - 1) / kSms]);
+    if (best_cost == 0.0 || cost < best_cost) {
+      best = tz;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+inline int stage_blocks(const FillBox& fb) { return stage_blocks(fb, stage_tz(fb)); }
+// the most blocks of any fill box inside `whole`
+inline int stage_blocks_max(const FillBox& whole) {
+  const int b = stage_blocks(whole, kStageMaxTZ);
+  return b > kStageMaxSplit ? b : kStageMaxSplit;
 }
 
 // kind: StageKind; prec: 8 (FP64) or 4 (FP32)
