@@ -77,6 +77,16 @@ __device__ __forceinline__ bool kless(const Time3& tx, long ix, const Time3& ty,
   if (tless(ty, tx)) return false;
   return ix < iy;
 }
+// the same out of line, for the rare comparisons of times whose first levels tie
+__device__ __noinline__ bool kless_tied(Time3 tx, long ix, Time3 ty, long iy) {
+  return kless(tx, ix, ty, iy);
+}
+
+// loads of values that other SMs write during the march: from L2, since an
+// L1 line may predate the write
+__device__ __forceinline__ Time3 ldcg(const Time3* t) {
+  return Time3{__ldcg(&t->a), __ldcg(&t->b), __ldcg(&t->c)};
+}
 
 // linear index of the k-th point (k = 1, 2) from o in slot q's direction
 __device__ __forceinline__ long nb_index(long o, const long s[3], int q, int k) {
@@ -223,6 +233,17 @@ __global__ void k_eik_front(double* d, Time3* tm, unsigned char* st, const doubl
   }
 }
 
+// A point's update: its value and acceptance time, and per axis what it took
+// (the side, -1: none; the value there; the next point's value where the
+// second-order stencil holds).
+struct Update {
+  double val;
+  Time3 t;
+  int side[3];
+  bool second[3];
+  double u1[3], u2[3];
+};
+
 // The neighbours of one point, by slot 2*axis + (plus side): the immediate
 // neighbour (value v1, time t1) and, at second order, the next one in that
 // direction (v2, t2).
@@ -311,14 +332,18 @@ __device__ __forceinline__ double fmm_root(double A, double B, double disc) {
 // the points whose stencil reads it for the next pass.  A point whose time
 // is above T keeps its time as a candidate and waits in a pending list;
 // when a pass queues nothing, T moves to max(T + delta, smallest
-// candidate) and the pending points it reaches are queued.  A pass is two
-// kernels: k_fmm_pass evaluates every queued point from the values before
-// the pass (and, after a threshold advance, moves the pending points the
-// new T reaches to the next queue), k_fmm_apply stores the changes, queues
-// their readers and runs the threshold control in its last block.
+// candidate) and the pending points it reaches are queued.  All passes run
+// in one kernel, k_fmm_march, whose blocks meet twice a pass: every queued
+// point is evaluated from the values before the pass and its readers queued;
+// then the changes are stored.
 
-// the threshold advances by this many of the smallest spacing per step
-constexpr double kDeltaCells = 2.0;
+// The threshold advances by this many of the smallest spacing per step.  A
+// longer step takes fewer passes and revises its points more often: 6 cells
+// where the lists leave threads idle and a pass costs its latency (301x237,
+// order 1: 571 passes of 10.5 us with 2 cells, 405 of 11.3 with 6; 64^3: 256
+// and 228 of 14.0), 2 where they fill the GPU (128x112x120, order 2: 16.8 ms
+// against 20.6 with 6).
+constexpr double kDeltaCells = 2.0, kDeltaCellsSmall = 6.0;
 
 // The value and acceptance time of free point o from its neighbours' current
 // values and times: the reference's last trial update.  Every front point is
@@ -335,12 +360,13 @@ constexpr double kDeltaCells = 2.0;
 // solver the point's input.  Neighbours off the grid
 // are left out, as the reference's bounds checks do.
 template <int ORDER, bool EIK>
-__device__ __forceinline__ bool fmm_point(const double* d, const Time3* tm,
-                                          const unsigned char* st, long o, const int c[3],
-                                          const int n[3], const long s[3], const double i2[3],
-                                          const Eik& E, Stencil& nb, double& val, Time3& tv,
-                                          int& incl_out, Time3& trig_out, long& itrig_out,
-                                          bool& trig_free_out) {
+__device__ __noinline__ bool fmm_point(const double* d, const Time3* tm, const unsigned char* st,
+                                       long o, int c0, int c1, int c2, int nx, int ny, int nz,
+                                       double i2x, double i2y, double i2z, Eik E, Update* U) {
+  const int c[3] = {c0, c1, c2}, n[3] = {nx, ny, nz};
+  const long s[3] = {1L, (long)nx, (long)nx * ny};
+  const double i2[3] = {i2x, i2y, i2z};
+  Stencil nb;
   // every load first, at in-range addresses (the point itself stands in
   // for a neighbour off the grid), so that they are in flight together
   unsigned char s1[6], s2[6];
@@ -352,14 +378,14 @@ __device__ __forceinline__ bool fmm_point(const double* d, const Time3* tm,
     in1[q] = c[dir] + sg >= 0 && c[dir] + sg < n[dir];
     const long o1 = in1[q] ? o + sg * s[dir] : o;
     s1[q] = st[o1];
-    nb.v1[q] = d[o1];
-    nb.t1[q] = tm[o1];
+    nb.v1[q] = __ldcg(d + o1);
+    nb.t1[q] = ldcg(tm + o1);
     if (ORDER == 2) {
       in2[q] = in1[q] && c[dir] + 2 * sg >= 0 && c[dir] + 2 * sg < n[dir];
       const long o2 = in2[q] ? o + 2 * sg * s[dir] : o;
       s2[q] = st[o2];
-      nb.v2[q] = d[o2];
-      nb.t2[q] = tm[o2];
+      nb.v2[q] = __ldcg(d + o2);
+      nb.t2[q] = ldcg(tm + o2);
     }
   }
   nb.has1 = nb.front1 = nb.has2 = nb.front2 = 0;
@@ -449,12 +475,26 @@ __device__ __forceinline__ bool fmm_point(const double* d, const Time3* tm,
       }
     }
     if (!bad) {
-      val = cur;
-      tv = t;
-      incl_out = incl;
-      trig_out = trig;
-      itrig_out = itrig;
-      trig_free_out = trig_free;
+      U->val = cur;
+      U->t = t;
+#pragma unroll
+      for (int dir = 0; dir < 3; dir++) {
+        U->side[dir] = -1;
+        U->second[dir] = false;
+        U->u1[dir] = U->u2[dir] = DBL_MAX;
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+          const int q = 2 * dir + side;
+          if (!(incl & (1 << q))) continue;
+          if (side == 1 && !(fabs(nb.v1[q]) < fabs(U->u1[dir]))) continue;
+          U->side[dir] = side;
+          U->u1[dir] = nb.v1[q];
+          U->second[dir] = ORDER == 2 && (nb.has2 & (1 << q)) && fabs(nb.v2[q]) <= fabs(nb.v1[q]) &&
+                           ((nb.front2 & (1 << q)) ||
+                            (trig_free && kless(nb.t2[q], nb_index(o, s, q, 2), trig, itrig)));
+          U->u2[dir] = U->second[dir] ? nb.v2[q] : DBL_MAX;
+        }
+      }
       return true;
     }
     cap = badt;
@@ -462,45 +502,210 @@ __device__ __forceinline__ bool fmm_point(const double* d, const Time3* tm,
   }
 }
 
+// fmm_point for nearly every point, without most of its work.  Of 26 M
+// evaluations (128x112x120, order 2) none was taken twice, 0.002 % met a
+// negative discriminant and 0.03 % a lowered time, but each took 2.6 roots (a
+// square root and a division) to decide which neighbours come before the
+// value, and some 3000 instructions in a row.  Here
+//   - only the first level of a time is read; the others when two tie;
+//   - "a neighbour of key x comes before |value|" is read off the sign of the
+//     quadratic at x where it is clear of rounding, and the root is taken once
+//     at the end;
+//   - whatever is unusual (a lowered or tied time of the point itself, a
+//     negative or undefined discriminant, a vanishing linear term, for the
+//     Eikonal solver a negative value) is left to fmm_point.
+// Returns 1 with the update, 0 for a point no neighbour reaches, -1 for a
+// point left to fmm_point.  The arithmetic of the coefficients and of the
+// root is fmm_coeffs' and fmm_root's.
+template <int ORDER, bool EIK>
+__device__ __forceinline__ int fmm_point_fast(const double* d, const Time3* tm,
+                                              const unsigned char* st, long o, const int c[3],
+                                              const int n[3], const long s[3],
+                                              const double i2[3], const Eik& E, Update& U) {
+  double v1[6], k1[6], v2[6], k2[6];
+  unsigned char s1[6], s2[6];
+  unsigned in1 = 0, in2 = 0;
+  const double cterm = EIK ? 1 / E.speed[o] / E.speed[o] : 1.0;
+  // every load first, at in-range addresses, as in fmm_point
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const int dir = q >> 1, sg = (q & 1) ? 1 : -1;
+    const int a1 = c[dir] + sg, a2 = c[dir] + 2 * sg;
+    const bool i1 = a1 >= 0 && a1 < n[dir];
+    const long o1 = i1 ? o + sg * s[dir] : o;
+    in1 |= (unsigned)i1 << q;
+    s1[q] = st[o1];
+    v1[q] = __ldcg(d + o1);
+    k1[q] = __ldcg(&tm[o1].a);
+    if (ORDER == 2) {
+      const bool b2 = a2 >= 0 && a2 < n[dir];
+      const long o2 = b2 ? o + 2 * sg * s[dir] : o;
+      in2 |= (unsigned)b2 << q;
+      s2[q] = st[o2];
+      v2[q] = __ldcg(d + o2);
+      k2[q] = __ldcg(&tm[o2].a);
+    }
+  }
+  // masks, a bit per slot: in the update so far (the fronts), waiting (the
+  // free neighbours, their keys in k1), the second point usable at once
+  // (a front) or once accepted before the trigger; a bit per axis: the plus
+  // side is the smaller
+  unsigned incl = 0, rem = 0, sec = 0, dyn = 0, plus_less = 0;
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const bool has = (in1 >> q & 1) && s1[q] != kOutside && fabs(v1[q]) <= DBL_MAX;
+    const bool front = has && s1[q] == kFront;
+    incl |= (unsigned)front << q;
+    rem |= (unsigned)(has && !front) << q;
+    if (!(has && !front)) k1[q] = INFINITY;
+    if (ORDER == 2) {
+      const bool has2 = has && (in2 >> q & 1) && s2[q] != kOutside &&
+                        fabs(v2[q]) <= fabs(v1[q]);
+      const bool front2 = has2 && s2[q] == kFront;
+      sec |= (unsigned)front2 << q;
+      dyn |= (unsigned)(has2 && !front2) << q;
+    }
+  }
+#pragma unroll
+  for (int dir = 0; dir < 3; dir++)
+    plus_less |= (unsigned)(fabs(v1[2 * dir + 1]) < fabs(v1[2 * dir])) << dir;
+  if (!(incl | rem)) return 0;
+  double trig = -INFINITY;   // key of the last free neighbour taken
+  int qtrig = -1;
+  double A = 0, B = 0, C = 0, disc = 0;
+  unsigned used = 0, plus = 0, second = 0;   // a bit per axis, of the update so far
+  for (;;) {
+    if (incl) {
+      unsigned now = sec;
+      if (ORDER == 2) {
+        unsigned tie = 0;
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+          now |= (dyn >> q & 1 & (unsigned)(k2[q] < trig)) << q;
+          tie |= (dyn >> q & 1 & (unsigned)(k2[q] == trig)) << q;
+        }
+        if (tie) {
+          const long it = nb_index(o, s, qtrig, 1);
+#pragma unroll
+          for (int q = 0; q < 6; q++)
+            if (tie >> q & 1) {
+              const long iq = nb_index(o, s, q, 2);
+              if (kless_tied(ldcg(tm + iq), iq, ldcg(tm + it), it)) now |= 1u << q;
+            }
+        }
+      }
+      used = plus = second = 0;
+      A = B = C = 0;
+#pragma unroll
+      for (int dir = 0; dir < 3; dir++) {
+        const unsigned m = incl >> (2 * dir) & 3;
+        const bool pl = m == 2 || (m == 3 && (plus_less >> dir & 1));
+        const double u1 = pl ? v1[2 * dir + 1] : v1[2 * dir];
+        const double inv = i2[dir];
+        double a, b, g;
+        if (ORDER == 1) {
+          a = inv;
+          b = inv * u1;
+          g = inv * u1 * u1;
+        } else {
+          const bool sw = now >> (2 * dir + pl) & 1;
+          const double u2 = pl ? v2[2 * dir + 1] : v2[2 * dir];
+          const double w = sw ? 1.5 : 1.0;
+          const double contrib = sw ? 2.0 * u1 - 0.5 * u2 : u1;
+          a = inv * w * w;
+          b = inv * w * contrib;
+          g = inv * contrib * contrib;
+          second |= (unsigned)sw << dir;
+        }
+        used |= (unsigned)(m != 0) << dir;
+        plus |= (unsigned)pl << dir;
+        // (x + 0 = x for the sums' values; an axis that is not used may hold anything)
+        A += m ? a : 0.0;
+        B += m ? b : 0.0;
+        C += m ? g : 0.0;
+      }
+      B *= -2.0;
+      C -= cterm;
+      disc = B * B - 4.0 * A * C;
+      if (!(disc >= 0) || !(fabs(B) > 1e-9) || (EIK && B > 0)) return -1;
+    }
+    if (!rem) break;
+    // the earliest remaining free neighbour
+    double x;
+    {
+      const double a = k1[0] < k1[1] ? k1[0] : k1[1], b = k1[2] < k1[3] ? k1[2] : k1[3],
+                   e = k1[4] < k1[5] ? k1[4] : k1[5];
+      x = a < b ? a : b;
+      x = x < e ? x : e;
+    }
+    unsigned eq = 0;
+#pragma unroll
+    for (int q = 0; q < 6; q++) eq |= (unsigned)(k1[q] == x) << q;
+    eq &= rem;
+    if (!eq) return -1;   // an undefined key
+    if (incl) {
+      // x against |value|, the outer root of A u^2 - |B| u + C
+      const double ax = A * x, bx = fabs(B);
+      const double f = (ax - bx) * x + C;
+      const double clear = 1e-12 * ((ax + bx) * x + fabs(C));
+      if (!(f < -clear)) {
+        if (f > clear && 2.0 * ax > bx) break;
+        const double r = fabs(fmm_root<EIK>(A, B, disc));
+        if (x > r) break;
+        if (!(x < r)) return -1;
+      }
+    }
+    if (eq & (eq - 1)) {   // equal keys: the whole times decide, then the indices
+      int best = -1;
+      for (unsigned m = eq; m; m &= m - 1) {
+        const int q = __ffs(m) - 1;
+        const long iq = nb_index(o, s, q, 1), ib = nb_index(o, s, best < 0 ? q : best, 1);
+        if (best < 0 || kless_tied(ldcg(tm + iq), iq, ldcg(tm + ib), ib)) best = q;
+      }
+      eq = 1u << best;
+    }
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+      if (eq >> q & 1) k1[q] = INFINITY;
+    rem &= ~eq;
+    incl |= eq;
+    trig = x;
+    qtrig = __ffs(eq) - 1;
+  }
+  U.val = fmm_root<EIK>(A, B, disc);
+  const double t = fabs(U.val);
+  if (!(t > trig)) return -1;
+  U.t = Time3{t, -1.0, -1.0};
+#pragma unroll
+  for (int dir = 0; dir < 3; dir++) {
+    const bool pl = plus >> dir & 1;
+    U.side[dir] = (used >> dir & 1) ? pl : -1;
+    U.second[dir] = ORDER == 2 && (second >> dir & 1);
+    U.u1[dir] = pl ? v1[2 * dir + 1] : v1[2 * dir];
+    U.u2[dir] = ORDER == 2 ? (pl ? v2[2 * dir + 1] : v2[2 * dir]) : DBL_MAX;
+  }
+  return 1;
+}
+
 // The extension fields of the point's last trial update: over the axes in
 // the update, the weighted average of the upwind neighbour's field with
 // weights (dist - phi_upwind)/dx^2, or (1.5 dist - 2 phi_upwind1 +
 // 0.5 phi_upwind2)/dx^2 where the second-order stencil is used
-// (lsm_FMM_field_extension.c:1135-1168, :1400-1460); ``val`` is the
+// (lsm_FMM_field_extension.c:1135-1168, :1400-1460); its value is the
 // update's distance (the previous one where the discriminant was
 // negative).  Each field whose value changes is stored; returns whether any
 // did.
-template <int ORDER>
-__device__ __forceinline__ bool fmm_ext(const Stencil& n, int incl, const Time3& trig,
-                                        long itrig, bool has_trigger, double val,
-                                        const double i2[3], const ExtSet& X, long o,
-                                        const long s[3]) {
+__device__ __forceinline__ bool fmm_ext(const Update& U, const double i2[3], const ExtSet& X,
+                                        long o, const long s[3]) {
   double g[3];
   long a[3];
   bool used[3];
 #pragma unroll
   for (int dir = 0; dir < 3; dir++) {
-    double u1 = DBL_MAX, u2 = DBL_MAX;
-    int sw = 0, side_used = -1;
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-      const int q = 2 * dir + side;
-      if (!(incl & (1 << q))) continue;
-      if (side == 1 && !(fabs(n.v1[q]) < fabs(u1))) continue;
-      u1 = n.v1[q];
-      u2 = DBL_MAX;
-      sw = 0;
-      side_used = side;
-      if (ORDER == 2 && (n.has2 & (1 << q)) && fabs(n.v2[q]) <= fabs(u1) &&
-          ((n.front2 & (1 << q)) ||
-           (has_trigger && kless(n.t2[q], nb_index(o, s, q, 2), trig, itrig)))) {
-        u2 = n.v2[q];
-        sw = 1;
-      }
-    }
-    used[dir] = side_used >= 0;
-    a[dir] = side_used == 1 ? o + s[dir] : o - s[dir];
-    g[dir] = (ORDER == 2 && sw == 1) ? 1.5 * val - 2.0 * u1 + 0.5 * u2 : val - u1;
+    used[dir] = U.side[dir] >= 0;
+    a[dir] = U.side[dir] == 1 ? o + s[dir] : o - s[dir];
+    g[dir] = U.second[dir] ? 1.5 * U.val - 2.0 * U.u1[dir] + 0.5 * U.u2[dir]
+                           : U.val - U.u1[dir];
   }
   bool changed = false;
 #pragma unroll
@@ -510,11 +715,11 @@ __device__ __forceinline__ bool fmm_ext(const Stencil& n, int incl, const Time3&
 #pragma unroll
     for (int dir = 0; dir < 3; dir++) {
       if (!used[dir]) continue;
-      num += i2[dir] * g[dir] * X.ext[f][a[dir]];
+      num += i2[dir] * g[dir] * __ldcg(X.ext[f] + a[dir]);
       den += i2[dir] * g[dir];
     }
     const double v = num / den;
-    if (__double_as_longlong(v) != __double_as_longlong(X.ext[f][o])) {
+    if (__double_as_longlong(v) != __double_as_longlong(__ldcg(X.ext[f] + o))) {
       X.ext[f][o] = v;
       changed = true;
     }
@@ -522,22 +727,21 @@ __device__ __forceinline__ bool fmm_ext(const Stencil& n, int incl, const Time3&
   return changed;
 }
 
-// Device state of the solve, read and advanced by the kernels so that the
-// host only launches and, every few passes, looks at ``done``.
+// Device words of the solve.  The counts and minima gather over one pass and
+// are read by every block after the barrier that ends it; three slots in
+// turn, so that a slot is cleared a pass before its next use, when no block
+// can still be reading it, and none adds to a slot that another reads.
 struct Ctrl {
-  int pass;                  // passes run so far
-  int count[2];              // lengths of the two active lists (by pass parity)
-  int pend_count[2];         // lengths of the two pending lists (by epoch parity)
-  int epoch;                 // number of threshold advances
-  int done;
-  int advance;               // the last control step moved the threshold
-  int filter_count;          // length of the pending list being filtered
-  int peak;                  // largest queue of the current threshold step
-  double T;                  // threshold on the first level of the time
-  unsigned long long minrej; // bits of the smallest candidate queued since
-                             // the last advance (times are >= 0)
-  unsigned long long minkeep;// bits of the smallest candidate kept waiting
-  int arrived;               // blocks of the current k_fmm_apply that finished
+  int count[3];              // length of the active list of pass p: slot p % 3
+  int pend_count[3];         // points pass p added to the pending list: slot p % 3
+  unsigned long long minrej[3];   // bits of the smallest candidate among them
+                                  // (times are >= 0),
+  unsigned long long minkeep[3];  // and of those kept waiting: slot p % 3
+  int pass;                  // result: passes run
+  int done;                  // result: converged
+  int error;                 // a barrier wait gave up
+  alignas(128) unsigned arrived;  // blocks at the barrier, counted up for good
+  alignas(128) unsigned released; // barriers passed
 };
 
 struct Lists {
@@ -545,9 +749,9 @@ struct Lists {
   int* stamp;                // pass that last queued a point
   int* pending;              // two lists of n points (by epoch parity)
   int* pend_stamp;           // epoch + 1 that last queued a point
-  double* new_d;             // per slot of the active list: the evaluated value,
-  Time3* new_t;              //   time and what to apply (bit 0: evaluated,
-  unsigned char* new_f;      //   bit 1: an extension field changed)
+  double* new_d;             // per slot of the active list beyond each thread's
+  Time3* new_t;              //   first: the evaluated value, time and whether
+  unsigned char* new_f;      //   to store them
 };
 
 // grid coordinates of point o (the entry points limit grids to 2^31 - 1
@@ -569,11 +773,6 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
   return v;
 }
 
-__device__ __forceinline__ void push_once(long p, int stamp_val, int* stamp, int* list,
-                                          int* count) {
-  if (atomicExch(stamp + p, stamp_val) != stamp_val) list[atomicAdd(count, 1)] = (int)p;
-}
-
 // The first active list: the free points next to the front.
 __global__ void k_fmm_seed(const unsigned char* st, int nx, int ny, int nz, Lists L,
                            Ctrl* ctrl) {
@@ -592,289 +791,370 @@ __global__ void k_fmm_seed(const unsigned char* st, int nx, int ny, int nz, List
       const int c1 = c[dir] + sg;
       if (c1 >= 0 && c1 < nn[dir] && st[o + sg * s[dir]] == kFront) near = true;
     }
-    if (near) push_once(o, 1, L.stamp, L.active, &ctrl->count[0]);
+    if (near) {
+      L.stamp[o] = 1;
+      L.active[atomicAdd(&ctrl->count[0], 1)] = (int)o;
+    }
   }
 }
 
-// The first half of a pass over the active list (count[pass & 1]): each
-// point's value and time from the values before the pass, into the list's
-// side arrays, with what changed; rejected points join the pending list.
-// After a threshold advance it also filters the last epoch's pending list
-// (below the main loop).
-template <int ORDER, bool EIK>
-__global__ void __launch_bounds__(128, ORDER == 1 ? 4 : 3)
-k_fmm_pass(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int nz,
-           double i2x, double i2y, double i2z, Lists L, Ctrl* ctrl, ExtSet X, Eik E) {
-  // the control words, and the first slot of both active lists (the pass
-  // number picks one), are loaded together: no load waits on another
+// Once the queued points fall to 1/kTailFraction of the threshold step's
+// largest pass, the threshold moves on.  Each step has a burst of large
+// passes and then a long tail of small ones as the last revisions settle;
+// the threshold need not wait for that tail (the fixed point does not
+// depend on when T moves, only the amount of revision does).  4 against 8:
+// 442 passes for 493 (128x112x120, order 1), the points up by a sixth, the
+// time down by 6 to 14 % over the sizes tried.
+constexpr int kTailFraction = 4;
+
+// Threads of a block of k_fmm_march, one block per SM (or of the one
+// cluster): 122 registers at order 1, 168 at order 2.
+__host__ __device__ constexpr int march_threads(int order) { return order == 1 ? 512 : 384; }
+constexpr int kClusterBlocks = 8;
+
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;   // +infinity
+
+// polls of a grid barrier before it gives up (seconds)
+constexpr int kBarrierPolls = 1 << 24;
+
+// Every block of the march has arrived (and its writes are visible) when
+// this returns.  One cluster: the hardware barrier.  Else the blocks of a
+// cooperative launch count themselves in and wait for the last one's word;
+// a wait that gives up sets ctrl->error and returns false to every thread.
+template <bool CLUSTER>
+__device__ __forceinline__ bool march_barrier(Ctrl* ctrl, unsigned& gen, int* s_ok) {
+  if constexpr (CLUSTER) {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  } else {
+    gen++;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int ok = 1;
+      __threadfence();
+      if (atomicAdd(&ctrl->arrived, 1u) == gen * gridDim.x - 1) {
+        __threadfence();
+        *(volatile unsigned*)&ctrl->released = gen;
+      } else {
+        int polls = 0;
+        while (*(volatile unsigned*)&ctrl->released < gen)
+          if (++polls == kBarrierPolls) {
+            *(volatile int*)&ctrl->error = 1;
+            ok = 0;
+            break;
+          }
+      }
+      __threadfence();
+      *s_ok = ok;
+    }
+    __syncthreads();
+    return *s_ok != 0;
+  }
+}
+
+// *p exchanged with v where the predicate holds, and the old value; v elsewhere
+__device__ __forceinline__ int exch_if(unsigned pred, int* p, int v) {
+  int old;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.b32 %0, %2;\n\t"
+      "@q atom.global.exch.b32 %0, [%1], %2;\n\t}"
+      : "=&r"(old)
+      : "l"(p), "r"(v), "r"(pred)
+      : "memory");
+  return old;
+}
+
+// This thread's points go to positions of two lists, `mine` (0..12) and
+// `mine2` (0 or 1) of them: the block reserves its room with one addition to
+// each list's length (same-address atomics of every warp of the grid took
+// longer than the evaluation).  Returns the thread's first position in each.
+// Every thread of the block takes part.
+struct Room {
+  int warp_at[2][16];
+  int base[2];
+};
+__device__ __forceinline__ int2 reserve(int mine, int mine2, int* count, int* count2, Room* r) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int upto = mine;
+#pragma unroll
+  for (int sh = 1; sh < 32; sh <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, upto, sh);
+    if (lane >= sh) upto += v;
+  }
+  const unsigned ones = __ballot_sync(0xffffffffu, mine2 != 0);
+  if (lane == 31) {
+    r->warp_at[0][wid] = upto;
+    r->warp_at[1][wid] = __popc(ones);
+  }
+  __syncthreads();
+  if (wid == 0) {
+    // lanes 0..15: the first list's warps, 16..31: the second's
+    const int half = lane >> 4, w = lane & 15;
+    int n = w < nw ? r->warp_at[half][w] : 0;
+    const int own = n;
+#pragma unroll
+    for (int sh = 1; sh < 16; sh <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, n, sh, 16);
+      if (w >= sh) n += v;
+    }
+    if (w < nw) r->warp_at[half][w] = n - own;
+    if (w == 15) r->base[half] = n ? atomicAdd(half ? count2 : count, n) : 0;
+  }
+  __syncthreads();
+  const int2 at = make_int2(r->base[0] + r->warp_at[0][wid] + upto - mine,
+                            r->base[1] + r->warp_at[1][wid] +
+                                __popc(ones & ((1u << lane) - 1u)));
+  __syncthreads();   // the words are free for the next call
+  return at;
+}
+
+// The whole march.  A pass p over its active list:
+//   - each point's value and time from the values before the pass (evaluated
+//     in place, while others change, a half-written neighbour can sustain
+//     an oscillation that sequential or synchronous sweeps never enter);
+//     rejected points join the pending list, the readers of a changed point
+//     the list of pass p + 1 (stamped p + 2);
+//   - after a threshold advance, the pending points of the last epoch that
+//     the new threshold reaches join that list too, the others wait in this
+//     epoch's pending list;
+//   - barrier; the changes are stored; barrier;
+//   - every block draws the same conclusion from the counts: the pass done,
+//     the threshold moved, or the march ended (nothing queued or waiting).
+// The passes are a chain of memory round trips over short lists (a few
+// thousand to some ten thousand points), so their number times the latency of
+// one is the time.  As two kernels a pass in a replayed graph, with a third
+// of the time between kernels, a pass took 17 to 20 us (128x112x120, order 2:
+// 24.9 ms a call from host arrays; 301x237, two extension fields: 11.9 ms).
+// Here the readers are queued by the thread that found the change, beside
+// the evaluation, a thread keeps its first slot's result in registers, the
+// stamps of a point's readers are exchanged together, and the warps of a
+// short list are spread over the SMs: 10 to 15 us a pass where the lists are
+// short (half of it the evaluation, the rest the two barriers and the queue),
+// 35 at 68,000 points a pass.
+// Lists that fit one cluster's threads run on 8 SMs, whose barrier is a
+// hardware one.
+template <int ORDER, bool EIK, bool CLUSTER>
+__global__ void __launch_bounds__(march_threads(ORDER), 1)
+k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int nz, double i2x,
+            double i2y, double i2z, Lists L, Ctrl* ctrl, ExtSet X, Eik E, double delta,
+            int max_passes) {
+  constexpr int kReaders = 6 * ORDER;
+  __shared__ Room room;
+  __shared__ unsigned long long s_min[2];
+  __shared__ struct {
+    int count, waiting, filter, ep, advance, done;
+    double T;
+  } c_;
+  __shared__ int s_ok;
   const long n = (long)nx * ny * nz;
-  const int w_first = blockIdx.x * blockDim.x + threadIdx.x;
-  const int first0 = w_first < n ? L.active[w_first] : 0;
-  const int first1 = w_first < n ? L.active[n + w_first] : 0;
-  const int it = ctrl->pass;
-  const int count0 = ctrl->count[0], count1 = ctrl->count[1];
-  const int ep = ctrl->epoch;
-  const double T = ctrl->T;
-  const int advance = ctrl->advance, filter_count = ctrl->filter_count;
-  const int par = it & 1;
-  const int count = par ? count1 : count0;
-  const int* cur = L.active + par * n;
-  int* pend = L.pending + (ep & 1) * n;
-  int* pend_count = &ctrl->pend_count[ep & 1];
+  const int lane = threadIdx.x & 31;
+  const int nb = (int)gridDim.x, bid = (int)blockIdx.x;
+  const int total = nb * (int)blockDim.x;
+  // slot of a round: warps go over the blocks first
+  const int slot = (((int)threadIdx.x >> 5) * nb + bid) * 32 + lane;
   const double i2[3] = {i2x, i2y, i2z};
   const int nn[3] = {nx, ny, nz};
   const long s[3] = {1L, (long)nx, (long)nx * ny};
-  unsigned long long minrej = ~0ULL;
-  for (int w = w_first; w < count; w += gridDim.x * blockDim.x) {
-    const long o = w == w_first ? (par ? first1 : first0) : cur[w];
-    // only free points are ever queued; the status, value and time of the
-    // point itself are loaded beside its stencil
-    const unsigned char self = st[o];
-    const double old = d[o];
-    const Time3 told = tm[o];
-    int c[3];
-    point_coords(o, nx, ny, c);
-    Stencil nb;
-    double val;
-    Time3 tv, trig;
-    long itrig;
-    int incl;
-    bool trig_free;
-    bool ext_changed = false;
-    const bool reached = fmm_point<ORDER, EIK>(d, tm, st, o, c, nn, s, i2, E, nb, val, tv,
-                                               incl, trig, itrig, trig_free);
-    if (self != kFree) {
-      L.new_f[w] = 0;
-      continue;
-    }
-    if (!reached) {
-      // no neighbour is reached (any more): no update, the point is unreached
-      val = copysign(INFINITY, old);
-      tv = Time3{INFINITY, INFINITY, INFINITY};
-    } else if (!(tv.a <= T)) {
-      // accepted after the threshold: a candidate only, waiting for T
-      val = copysign(INFINITY, old);
-      push_once(o, ep + 1, L.pend_stamp, pend, pend_count);
-      const unsigned long long bits = __double_as_longlong(tv.a);
-      minrej = bits < minrej ? bits : minrej;
-    } else if (!EIK && X.nf) {
-      ext_changed = fmm_ext<ORDER>(nb, incl, trig, itrig, trig_free, val, i2, X, o, s);
-    }
-    // what k_fmm_apply does with the slot: bit 0 store the value and time,
-    // bit 1 queue the readers (the change is visible: the value is finite
-    // before or after, or an extension field changed)
-    unsigned char f = 0;
-    if (ext_changed || !(val == old && tequal(tv, told))) {
-      f = 1;
-      if (ext_changed || fabs(old) <= DBL_MAX || fabs(val) <= DBL_MAX) f |= 2;
-    }
-    L.new_d[w] = val;
-    L.new_t[w] = tv;
-    L.new_f[w] = f;
+  unsigned gen = 0;
+  // thread 0: the largest queue of the threshold step, its smallest candidate
+  int peak = 0;
+  unsigned long long smallest = kInfBits;
+  if (threadIdx.x == 0) {
+    c_.count = __ldcg(&ctrl->count[0]);
+    c_.T = delta;
+    c_.ep = c_.waiting = c_.filter = c_.advance = c_.done = 0;
+    s_min[0] = s_min[1] = kInfBits;
   }
-  minrej = warp_min(minrej);
-  if ((threadIdx.x & 31) == 0 && minrej != ~0ULL) atomicMin(&ctrl->minrej, minrej);
-  // After a threshold advance (the control step that ended the last pass):
-  // the pending points of the last epoch that the new threshold reaches join
-  // the queue of the next pass beside the readers k_fmm_apply queues (same
-  // list, same stamp); the others wait in this epoch's pending list.  Values
-  // and times do not change during this kernel, so the test reads them as
-  // the pass does.
-  if (advance) {
+  __syncthreads();
+  int pass = 0;
+  for (; pass < max_passes; pass++) {
+    const int count = c_.count, ep = c_.ep;
+    const double T = c_.T;
+    const int* cur = L.active + (pass & 1) * n;
+    int* next = L.active + ((pass + 1) & 1) * n;
+    int* next_count = &ctrl->count[(pass + 1) % 3];
+    int* pend = L.pending + (ep & 1) * n + c_.waiting;
+    int* pend_count = &ctrl->pend_count[pass % 3];
+    if (bid == 0 && threadIdx.x == 0) {
+      ctrl->count[(pass + 2) % 3] = 0;
+      ctrl->pend_count[(pass + 1) % 3] = 0;
+      ctrl->minrej[(pass + 1) % 3] = ctrl->minkeep[(pass + 1) % 3] = kInfBits;
+    }
+    unsigned long long minrej = kInfBits, minkeep = kInfBits;
+    // the first slot's result
+    bool f_first = false;
+    int o_first = 0;
+    double d_first = 0;
+    Time3 t_first{0, 0, 0};
+    for (int base = 0; base + bid * 32 < count; base += total) {
+      const int w = base + slot;
+      unsigned won = 0;
+      bool wait = false;
+      long o = 0;
+      if (w < count) {
+        o = __ldcg(cur + w);
+        // only free points are ever queued; the value and time of the
+        // point itself are loaded beside its stencil
+        const double old = __ldcg(d + o);
+        const Time3 told = ldcg(tm + o);
+        int c[3];
+        point_coords(o, nx, ny, c);
+        Update U;
+        int reached = fmm_point_fast<ORDER, EIK>(d, tm, st, o, c, nn, s, i2, E, U);
+        if (reached < 0) {
+          Update slow;
+          reached = fmm_point<ORDER, EIK>(d, tm, st, o, c[0], c[1], c[2], nx, ny, nz, i2x, i2y,
+                                          i2z, E, &slow);
+          U = slow;
+        }
+        double val = U.val;
+        Time3 tv = U.t;
+        bool ext_changed = false;
+        if (!reached) {
+          // no neighbour is reached (any more): no update, the point is unreached
+          val = copysign(INFINITY, old);
+          tv = Time3{INFINITY, INFINITY, INFINITY};
+        } else if (!(tv.a <= T)) {
+          // accepted after the threshold: a candidate only, waiting for T
+          val = copysign(INFINITY, old);
+          wait = atomicExch(L.pend_stamp + o, ep + 1) != ep + 1;
+          const unsigned long long bits = __double_as_longlong(tv.a);
+          minrej = bits < minrej ? bits : minrej;
+        } else if (!EIK && X.nf) {
+          ext_changed = fmm_ext(U, i2, X, o, s);
+        }
+        const bool store = ext_changed || !(val == old && tequal(tv, told));
+        if (base == 0) {
+          f_first = store;
+          o_first = (int)o;
+          d_first = val;
+          t_first = tv;
+        } else {
+          L.new_f[w] = store;
+          L.new_d[w] = val;
+          L.new_t[w] = tv;
+        }
+        // the free points whose stencil reads this one, where the change is
+        // visible: the value is finite before or after, or a field changed
+        if (store && (ext_changed || fabs(old) <= DBL_MAX || fabs(val) <= DBL_MAX)) {
+          unsigned cand = 0;
+#pragma unroll
+          for (int q = 0; q < 6; q++) {
+            const int dir = q >> 1, sg = (q & 1) ? 1 : -1;
+#pragma unroll
+            for (int r = 1; r <= ORDER; r++) {
+              const int cr = c[dir] + r * sg;
+              if (cr >= 0 && cr < nn[dir] && st[o + r * sg * s[dir]] == kFree)
+                cand |= 1u << (q * ORDER + r - 1);
+            }
+          }
+          // the exchanges go out together: predicated, without branches
+          int was[kReaders];
+#pragma unroll
+          for (int k = 0; k < kReaders; k++)
+            was[k] = exch_if(cand >> k & 1, L.stamp + nb_index(o, s, k / ORDER, k % ORDER + 1),
+                             pass + 2);
+#pragma unroll
+          for (int k = 0; k < kReaders; k++)
+            if (was[k] != pass + 2) won |= 1u << k;
+        }
+      }
+      const int2 at = reserve(__popc(won), wait, next_count, pend_count, &room);
+      if (wait) pend[at.y] = (int)o;
+      int pos = at.x;
+#pragma unroll
+      for (int k = 0; k < kReaders; k++)
+        if (won >> k & 1) next[pos++] = (int)nb_index(o, s, k / ORDER, k % ORDER + 1);
+    }
+    // the pending points of the last epoch after a threshold advance.  Values
+    // and times do not change before the barrier, so the test reads them as
+    // the pass does.
+    const int filter = c_.advance ? c_.filter : 0;
     const int* src = L.pending + ((ep - 1) & 1) * n;
-    int* next = L.active + (par ^ 1) * n;
-    unsigned long long mk = ~0ULL;
-    for (int w = w_first; w < filter_count; w += gridDim.x * blockDim.x) {
-      const long o = src[w];
-      if (fabs(d[o]) <= DBL_MAX) continue;   // reached since
-      const double t = tm[o].a;
-      if (t <= T) {
-        push_once(o, it + 2, L.stamp, next, &ctrl->count[par ^ 1]);
-      } else if (t < INFINITY) {
-        push_once(o, ep + 1, L.pend_stamp, pend, pend_count);
-        const unsigned long long bits = __double_as_longlong(t);
-        mk = bits < mk ? bits : mk;
-      }
-    }
-    mk = warp_min(mk);
-    if ((threadIdx.x & 31) == 0 && mk != ~0ULL) atomicMin(&ctrl->minkeep, mk);
-  }
-}
-
-// Between passes (the last block of k_fmm_apply, one thread).  Each
-// threshold step has a burst of large passes and then a long tail of small
-// ones as the last revisions settle; the threshold need not wait for that
-// tail (the fixed point does not depend on when T moves, only the amount of
-// revision does).  So once the queued points fall to 1/kTailFraction of the
-// step's largest pass, the threshold moves to max(T + delta, smallest
-// waiting candidate) and the pending list is filtered (by the next pass
-// kernel) into the queue after it.  With nothing queued and nothing waiting, the solve is
-// done.  The words are read volatile: other blocks of the same launch wrote
-// the queue length.
-constexpr int kTailFraction = 8;
-
-__device__ void fmm_control(double delta, volatile Ctrl* ctrl) {
-  // every word in one round of loads (none waits on another)
-  const int done = ctrl->done, pass = ctrl->pass, peak0 = ctrl->peak, ep = ctrl->epoch;
-  const int count0 = ctrl->count[0], count1 = ctrl->count[1];
-  const int pend0 = ctrl->pend_count[0], pend1 = ctrl->pend_count[1];
-  const unsigned long long rej = ctrl->minrej, keep = ctrl->minkeep;
-  const double T = ctrl->T;
-  if (done) return;
-  const int par = pass & 1;
-  const int queued = par ? count0 : count1;
-  const int peak = queued > peak0 ? queued : peak0;
-  int advance = 0;
-  if ((long)queued * kTailFraction <= peak) {
-    const int np = (ep & 1) ? pend1 : pend0;
-    if (np == 0) {
-      if (queued == 0) ctrl->done = 1;
-    } else {
-      const unsigned long long m = rej < keep ? rej : keep;
-      const double lo = __longlong_as_double((long long)m);
-      const double step = T + delta;
-      ctrl->T = lo > step ? lo : step;
-      advance = 1;
-      ctrl->filter_count = np;
-      ctrl->pend_count[(ep & 1) ^ 1] = 0;
-      ctrl->epoch = ep + 1;
-      ctrl->minrej = __double_as_longlong(INFINITY);
-      ctrl->minkeep = __double_as_longlong(INFINITY);
-    }
-  }
-  ctrl->peak = advance ? queued : peak;
-  ctrl->advance = advance;
-  ctrl->count[par] = 0;
-  ctrl->pass = pass + 1;
-}
-
-// The second half of a pass: the values and times evaluated by k_fmm_pass are
-// stored, and the points whose stencil reads a changed point are queued.
-// Evaluating every point of a pass from the values before it (rather than
-// in place, while others change) keeps the passes from cycling: read in
-// place, a half-written neighbour can sustain an oscillation that sequential
-// or synchronous sweeps never enter.
-//
-// The kernel is a short chain of memory round trips, so it is laid out to
-// keep each round in flight at once: a warp takes 32 consecutive slots; the
-// slot words load together; the readers' statuses load together; their
-// stamps are exchanged together; and the warp reserves its queue entries
-// with one atomic.  The block that finishes last runs the threshold control.
-template <int ORDER>
-__global__ void __launch_bounds__(256)
-k_fmm_apply(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int nz, Lists L,
-            Ctrl* ctrl, double delta) {
-  constexpr int kReaders = 6 * ORDER;
-  const long n = (long)nx * ny * nz;
-  const int lane = threadIdx.x & 31;
-  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  // the words of the first slot (both active lists for the point: the pass
-  // number picks one) load beside the control words
-  const int w_first = warp * 32 + lane;
-  unsigned char f_first = 0;
-  int first0 = 0, first1 = 0;
-  double d_first = 0;
-  Time3 t_first{0, 0, 0};
-  if (w_first < n) {
-    f_first = L.new_f[w_first];
-    first0 = L.active[w_first];
-    first1 = L.active[n + w_first];
-    d_first = L.new_d[w_first];
-    t_first = L.new_t[w_first];
-  }
-  const int it = ctrl->pass;
-  const int count0 = ctrl->count[0], count1 = ctrl->count[1];
-  const int par = it & 1;
-  const int count = par ? count1 : count0;
-  const int* cur = L.active + par * n;
-  int* next = L.active + (par ^ 1) * n;
-  int* next_count = &ctrl->count[par ^ 1];
-  const int nn[3] = {nx, ny, nz};
-  const long s[3] = {1L, (long)nx, (long)nx * ny};
-  // the loop bound is the same for the 32 lanes of a warp
-  for (int w0 = warp * 32; w0 < count; w0 += nwarps * 32) {
-    const int w = w0 + lane;
-    unsigned char f = 0;
-    long o = 0;
-    double val = 0;
-    Time3 tv{0, 0, 0};
-    if (w < count) {
-      if (w == w_first) {
-        f = f_first;
-        o = par ? first1 : first0;
-        val = d_first;
-        tv = t_first;
-      } else {
-        f = L.new_f[w];
-        o = cur[w];
-        val = L.new_d[w];
-        tv = L.new_t[w];
-      }
-    }
-    if (f & 1) {
-      d[o] = val;
-      tm[o] = tv;
-    }
-    // the free points whose stencil reads this one
-    long on[kReaders];
-    unsigned won = 0;
-    if (f & 2) {
-      int c[3];
-    point_coords(o, nx, ny, c);
-      unsigned char sn[kReaders];
-      unsigned cand = 0;
-#pragma unroll
-      for (int q = 0; q < 6; q++) {
-        const int dir = q >> 1, sg = (q & 1) ? 1 : -1;
-#pragma unroll
-        for (int r = 1; r <= ORDER; r++) {
-          const int k = q * ORDER + r - 1;
-          const int cr = c[dir] + r * sg;
-          const bool in = cr >= 0 && cr < nn[dir];
-          on[k] = in ? o + r * sg * s[dir] : o;
-          sn[k] = st[on[k]];
-          if (in) cand |= 1u << k;
+    for (int base = 0; base + bid * 32 < filter; base += total) {
+      const int w = base + slot;
+      bool go = false, wait = false;
+      int o = 0;
+      if (w < filter) {
+        o = __ldcg(src + w);
+        const double t = __ldcg(&tm[o].a);
+        if (!(fabs(__ldcg(d + o)) <= DBL_MAX)) {   // not reached since
+          if (t <= T) {
+            go = atomicExch(L.stamp + o, pass + 2) != pass + 2;
+          } else if (t < INFINITY) {
+            wait = atomicExch(L.pend_stamp + o, ep + 1) != ep + 1;
+            const unsigned long long bits = __double_as_longlong(t);
+            minkeep = bits < minkeep ? bits : minkeep;
+          }
         }
       }
-      int old[kReaders];
-#pragma unroll
-      for (int k = 0; k < kReaders; k++)
-        if ((cand >> k & 1) && sn[k] == kFree) {
-          old[k] = atomicExch(L.stamp + on[k], it + 2);
-          if (old[k] != it + 2) won |= 1u << k;
+      const int2 at = reserve(go, wait, next_count, pend_count, &room);
+      if (go) next[at.x] = o;
+      if (wait) pend[at.y] = o;
+    }
+    minrej = warp_min(minrej);
+    minkeep = warp_min(minkeep);
+    if (lane == 0) {
+      if (minrej != kInfBits) atomicMin(&s_min[0], minrej);
+      if (minkeep != kInfBits) atomicMin(&s_min[1], minkeep);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (s_min[0] != kInfBits) atomicMin(&ctrl->minrej[pass % 3], s_min[0]);
+      if (s_min[1] != kInfBits) atomicMin(&ctrl->minkeep[pass % 3], s_min[1]);
+      s_min[0] = s_min[1] = kInfBits;
+    }
+    if (!march_barrier<CLUSTER>(ctrl, gen, &s_ok)) return;
+    if (f_first) {
+      d[o_first] = d_first;
+      tm[o_first] = t_first;
+    }
+    for (int w = slot + total; w < count; w += total)
+      if (L.new_f[w]) {
+        const int o = __ldcg(cur + w);
+        d[o] = L.new_d[w];
+        tm[o] = L.new_t[w];
+      }
+    if (!march_barrier<CLUSTER>(ctrl, gen, &s_ok)) return;
+    // thread 0 of each block: the threshold control, from the same words in
+    // every block
+    if (threadIdx.x == 0) {
+      const int queued = __ldcg(next_count), np = c_.waiting + __ldcg(pend_count);
+      const unsigned long long rej = __ldcg(&ctrl->minrej[pass % 3]),
+                               keep = __ldcg(&ctrl->minkeep[pass % 3]);
+      smallest = rej < smallest ? rej : smallest;
+      smallest = keep < smallest ? keep : smallest;
+      peak = queued > peak ? queued : peak;
+      c_.waiting = np;
+      c_.advance = 0;
+      if ((long)queued * kTailFraction <= peak) {
+        if (np == 0) {
+          if (queued == 0) c_.done = 1;
+        } else {
+          const double lo = __longlong_as_double((long long)smallest);
+          const double step = T + delta;
+          c_.T = lo > step ? lo : step;
+          c_.advance = 1;
+          c_.filter = np;
+          c_.waiting = 0;
+          c_.ep = ep + 1;
+          peak = queued;
+          smallest = kInfBits;
         }
+      }
+      c_.count = queued;
     }
-    // one reservation for the warp's new queue entries
-    const int mine = __popc(won);
-    int upto = mine;
-#pragma unroll
-    for (int sh = 1; sh < 32; sh <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, upto, sh);
-      if (lane >= sh) upto += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, upto, 31);
-    if (total) {
-      int base = 0;
-      if (lane == 31) base = atomicAdd(next_count, total);
-      base = __shfl_sync(0xffffffffu, base, 31);
-      int pos = base + upto - mine;
-#pragma unroll
-      for (int k = 0; k < kReaders; k++)
-        if (won >> k & 1) next[pos++] = (int)on[k];
+    __syncthreads();
+    if (c_.done) {
+      pass++;
+      break;
     }
   }
-  // the last block to finish runs the control step
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0)
-    last = atomicAdd(&ctrl->arrived, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    __threadfence();
-    fmm_control(delta, ctrl);
-    ctrl->arrived = 0;
+  if (bid == 0 && threadIdx.x == 0) {
+    ctrl->pass = pass;
+    ctrl->done = c_.done;
   }
 }
 
@@ -899,13 +1179,15 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
   const int nx = grid_dims[0], ny = grid_dims[1], nz = grid_dims[2];
   const long n = (long)nx * ny * nz;
   const double hmin = fmin(dx[0], fmin(dx[1], dx[2]));
-  const double delta = kDeltaCells * hmin;
   // a bound on the passes for inputs without a fixed point (NaN): the
   // threshold crosses the grid in at most (diagonal / delta) steps of a
   // few passes each
   const long max_passes = 4096 + 32L * (nx + ny + nz);
   unsigned char* status = nullptr;
   Time3* tm = nullptr;
+  // points of a typical list: two per point of the grid's largest cross-section
+  const int longest = nx > ny ? (nx > nz ? nx : nz) : (ny > nz ? ny : nz);
+  const long band = 2 * n / longest;
   Lists L{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   Ctrl* ctrl = nullptr;
   const size_t un = (size_t)n;
@@ -920,9 +1202,7 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
             cuda_ok(pool_alloc((void**)&L.new_f, un, st), R) &&
             cuda_ok(pool_alloc((void**)&ctrl, sizeof(Ctrl), st), R);
   Ctrl h_ctrl{};
-  h_ctrl.T = delta;
-  h_ctrl.minrej = 0x7ff0000000000000ULL;   // +infinity
-  h_ctrl.minkeep = 0x7ff0000000000000ULL;
+  for (int q = 0; q < 3; q++) h_ctrl.minrej[q] = h_ctrl.minkeep[q] = kInfBits;
   int sms = 148;
   {
     int dev = 0;
@@ -953,62 +1233,52 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     i2[q] = 1 / dx[q];
     i2[q] *= i2[q];
   }
-  // a pass touches only the band, so a few blocks per SM cover it; the
-  // grid-stride loops take any count
-  const int pass_blocks = 4 * sms, apply_blocks = 2 * sms;
-  const int batch = 32;
-  auto launch_batch = [&](cudaStream_t s) {
-    for (int q = 0; q < batch; q++) {
-      if (order == 1 && !E.speed)
-        k_fmm_pass<1, false><<<pass_blocks, 128, 0, s>>>(dd, tm, status, nx, ny, nz, i2[0],
-                                                         i2[1], i2[2], L, ctrl, X, E);
-      else if (!E.speed)
-        k_fmm_pass<2, false><<<pass_blocks, 128, 0, s>>>(dd, tm, status, nx, ny, nz, i2[0],
-                                                         i2[1], i2[2], L, ctrl, X, E);
-      else if (order == 1)
-        k_fmm_pass<1, true><<<pass_blocks, 128, 0, s>>>(dd, tm, status, nx, ny, nz, i2[0],
-                                                        i2[1], i2[2], L, ctrl, X, E);
-      else
-        k_fmm_pass<2, true><<<pass_blocks, 128, 0, s>>>(dd, tm, status, nx, ny, nz, i2[0],
-                                                        i2[1], i2[2], L, ctrl, X, E);
-      if (order == 1)
-        k_fmm_apply<1><<<apply_blocks, 256, 0, s>>>(dd, tm, status, nx, ny, nz, L, ctrl,
-                                                     delta);
-      else
-        k_fmm_apply<2><<<apply_blocks, 256, 0, s>>>(dd, tm, status, nx, ny, nz, L, ctrl,
-                                                     delta);
-    }
-  };
-  // The kernels read the pass number and lists from ``ctrl``, so every batch
-  // is the same sequence of launches: capture it once as a CUDA graph and
-  // replay it (direct launches if the graph cannot be built).
-  cudaGraphExec_t gexec = nullptr;
+  // One cluster while the lists fit its threads, else one block per SM of a
+  // cooperative launch; and the threshold's step
+  const bool cluster = band <= kClusterBlocks * march_threads(2);
+  const bool small = cluster || 4 * band <= (long)sms * march_threads(order);
+  const double delta = (small ? kDeltaCellsSmall : kDeltaCells) * hmin;
+  // (passes in whole batches of 32)
+  int passes = (int)((max_passes + 31) / 32 * 32);
   if (ok) {
-    cudaStream_t cs = nullptr;
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess) {
-      if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        launch_batch(cs);
-        if (cudaStreamEndCapture(cs, &graph) == cudaSuccess && graph) {
-          if (cudaGraphInstantiate(&gexec, graph, 0) != cudaSuccess) gexec = nullptr;
-          cudaGraphDestroy(graph);
-        }
-      }
-      cudaStreamDestroy(cs);
+    const void* fn = nullptr;
+#define MARCH(O, K, C) (const void*)k_fmm_march<O, K, C>
+    if (order == 1)
+      fn = E.speed ? (cluster ? MARCH(1, true, true) : MARCH(1, true, false))
+                   : (cluster ? MARCH(1, false, true) : MARCH(1, false, false));
+    else
+      fn = E.speed ? (cluster ? MARCH(2, true, true) : MARCH(2, true, false))
+                   : (cluster ? MARCH(2, false, true) : MARCH(2, false, false));
+#undef MARCH
+    ExtSet xs = X;
+    Eik es = E;
+    double step = delta;
+    int mx = nx, my = ny, mz = nz;
+    void* args[] = {&dd, &tm, &status, &mx, &my,   &mz,   &i2[0], &i2[1],
+                    &i2[2], &L, &ctrl,   &xs, &es, &step, &passes};
+    cudaLaunchAttribute at{};
+    at.id = cluster ? cudaLaunchAttributeClusterDimension : cudaLaunchAttributeCooperative;
+    if (cluster) {
+      at.val.clusterDim.x = kClusterBlocks;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    } else {
+      at.val.cooperative = 1;
     }
-    cudaGetLastError();   // a failed capture leaves nothing behind but the error
-  }
-  long launched = 0;
-  while (ok) {
-    if (gexec) ok = cuda_ok(cudaGraphLaunch(gexec, st), R);
-    else launch_batch(st);
-    launched += batch;
-    launch_counter() += 2 * batch;
-    ok = ok && cuda_ok(cudaGetLastError(), R) &&
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster ? kClusterBlocks : sms);
+    cfg.blockDim = dim3(march_threads(order));
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    ok = cuda_ok(cudaLaunchKernelExC(&cfg, fn, args), R);
+    ++launch_counter();
+    ok = ok &&
          cuda_ok(cudaMemcpyAsync(&h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st), R) &&
          cuda_ok(cudaStreamSynchronize(st), R);
-    if (!ok || h_ctrl.done) break;
-    if (launched >= max_passes) {
+    if (ok && h_ctrl.error) {
+      set_error(LSMGPU_ERR_DEVICE, std::string(R) + ": a wait between blocks gave up");
+      ok = false;
+    } else if (ok && !h_ctrl.done) {
       set_error(LSMGPU_ERR_INVALID_VALUE, std::string(R) + ": no convergence (NaN in phi?)");
       ok = false;
     }
@@ -1018,7 +1288,6 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     ++launch_counter();
     ok = cuda_ok(cudaGetLastError(), R);
   }
-  if (gexec) cudaGraphExecDestroy(gexec);
   for (void* q : {(void*)status, (void*)tm, (void*)L.active, (void*)L.pending,
                   (void*)L.stamp, (void*)L.pend_stamp, (void*)L.new_d, (void*)L.new_t,
                   (void*)L.new_f, (void*)ctrl})
