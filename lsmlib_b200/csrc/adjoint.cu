@@ -546,7 +546,8 @@ struct lsmgpu_adjoint {
   double* theta = nullptr;
   double* grad_theta = nullptr;
   double* target = nullptr;
-  double* phi = nullptr;        // working state
+  double* phi0 = nullptr;       // the initial state as given, ghost cells included
+  double* phi = nullptr;        // final state
   double* s1 = nullptr;         // stage buffers
   double* s2 = nullptr;
   std::vector<double*> ckpt;    // checkpoint states
@@ -596,6 +597,9 @@ StageArgs fwd_args(lsmgpu_adjoint* h) {
   a.dx_sq = m * m;
   a.dt = h->dt;
   for (int d = 0; d < 3; d++) a.aux[d] = h->vel[d];
+  // every stage input is one of the problem's own buffers: its ghost cells
+  // take the boundary values (checkpoint 0 holds a copy of the caller's phi0)
+  a.ghosts_writable = 1;
   return a;
 }
 
@@ -703,17 +707,19 @@ bool loss_to_host(lsmgpu_adjoint* h, double* loss, cudaStream_t st, const char* 
   return true;
 }
 
-// forward run from phi0 (h->ckpt[0] holds phi0 after set_fields), storing the
-// checkpoints; the final state is left in h->phi
+// forward run from phi0 (h->ckpt[0] holds its interior), each step writing
+// straight into the next checkpoint where there is one; the final state is
+// left in h->phi, whose ghost cells are phi0's
 cudaError_t forward_run(lsmgpu_adjoint* h, cudaStream_t st) {
-  cudaError_t e = cudaMemcpyAsync(h->phi, h->ckpt[0], h->bytes, cudaMemcpyDeviceToDevice, st);
+  cudaError_t e = cudaMemcpyAsync(h->phi, h->phi0, h->bytes, cudaMemcpyDeviceToDevice, st);
   if (e) return e;
+  double* const work = h->lam2;   // scratch of the reverse sweep
   for (int s = 0; s < h->nsteps; s++) {
-    if (s % h->every == 0 && s > 0)
-      if ((e = cudaMemcpyAsync(h->ckpt[s / h->every], h->phi, h->bytes,
-                               cudaMemcpyDeviceToDevice, st)))
-        return e;
-    if ((e = fwd_step(h, h->phi, h->phi, st))) return e;
+    const double* in = s % h->every == 0 ? h->ckpt[s / h->every] : work;
+    double* out = s + 1 == h->nsteps          ? h->phi
+                  : (s + 1) % h->every == 0 ? h->ckpt[(s + 1) / h->every]
+                                            : work;
+    if ((e = fwd_step(h, out, in, st))) return e;
   }
   return cudaSuccess;
 }
@@ -764,6 +770,7 @@ int lsmgpu_adjoint_create(lsmgpu_adjoint** out, const int n[3], const double dx[
   h->theta = dalloc(3 * m3 * sizeof(double), ok);
   h->grad_theta = dalloc(3 * m3 * sizeof(double), ok);
   h->target = dalloc(h->bytes, ok);
+  h->phi0 = dalloc(h->bytes, ok);
   h->phi = dalloc(h->bytes, ok);
   h->s1 = dalloc(h->bytes, ok);
   h->s2 = dalloc(h->bytes, ok);
@@ -794,7 +801,7 @@ int lsmgpu_adjoint_create(lsmgpu_adjoint** out, const int n[3], const double dx[
 int lsmgpu_adjoint_destroy(lsmgpu_adjoint* h) {
   if (!h) return LSMGPU_SUCCESS;
   double* ps[] = {h->vel[0], h->vel[1], h->vel[2], h->A[0], h->A[1], h->A[2],
-                  h->theta, h->grad_theta, h->target, h->phi, h->s1, h->s2,
+                  h->theta, h->grad_theta, h->target, h->phi0, h->phi, h->s1, h->s2,
                   h->lam, h->lam2, h->lam1, h->T, h->Tb, h->partials};
   for (double* p : ps)
     if (p) cudaFree(p);
@@ -879,8 +886,10 @@ int lsmgpu_adjoint_set_fields(lsmgpu_adjoint* h, const double* phi0,
   }
   h->eps = eps;
   cudaStream_t st = cur_stream();
-  return cuda_ok(cudaMemcpyAsync(h->ckpt[0], phi0, h->bytes, cudaMemcpyHostToDevice, st),
-                 R) &&
+  return cuda_ok(cudaMemcpyAsync(h->phi0, phi0, h->bytes, cudaMemcpyHostToDevice, st), R) &&
+                 cuda_ok(cudaMemcpyAsync(h->ckpt[0], h->phi0, h->bytes,
+                                         cudaMemcpyDeviceToDevice, st),
+                         R) &&
                  cuda_ok(cudaMemcpyAsync(h->target, target, h->bytes,
                                          cudaMemcpyHostToDevice, st),
                          R) &&
