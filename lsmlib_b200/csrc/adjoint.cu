@@ -35,104 +35,95 @@ using namespace lsmgpu;
 
 namespace {
 
-// tile of k_adjoint_stage: kTX x kTY cells per block, kTZ planes per block
-// (build-time setting).  Short tiles balance the SMs: at 128^3 with two
-// blocks per SM, 32-plane tiles make 256 blocks (108 SMs with two, 40 with
-// one); 8-plane tiles make 1024 (about 7 per SM).  Measured reverse sweep of
-// the 128^3 problem: 207.1 ms (32 planes), 201.9 (16), 200.8 (8).
-#ifndef LSMGPU_ADJ_TZ
-#define LSMGPU_ADJ_TZ 8
-#endif
-constexpr int kTX = 32, kTY = 8, kTZ = LSMGPU_ADJ_TZ;
+// tile of k_adjoint_stage: kTX x kTY cells per block, adj_tz planes
+constexpr int kTX = 32, kTY = 8;
 
 // ---------------------------------------------------------------------------
-// one-sided WENO5 value and its gradient with respect to v1..v5
-//   D = sum w_k p_k,  w_k = a_k / sum a,  a_k = d_k / (S_k + eps)^2
-//   dD/dv = sum w_k dp_k + sum b_k (dS_k + deps),
-//   b_k = -2 w_k (p_k - D) / (S_k + eps)
-// The weights use the single-reciprocal normalisation of the forward stage
-// kernels (weno_fast.cuh): q_k = (S_k + eps) s with s a power of two,
-// w_k = d_k prod_{j!=k} q_j^2 / sum_m (...), and the three 1/(S_k + eps)
-// come from one more reciprocal, 1/q_k = s prod_{j!=k} q_j / (q_1 q_2 q_3).
+// One-sided WENO5 value and its gradient with respect to the six stencil
+// values W[0..5], in units of the undivided differences U_j = W[j] - W[j-1]
+// (the value is F(U) / dx; F is homogeneous of degree one):
+//   F = p2 + w1 (p1 - p2) + w3 (p3 - p2),  w_k = a_k / sum a,
+//   a_k = d_k / q_k^2,  q_k = S_k + eps,
+//   dF = dp2 + w1 d(p1 - p2) + w3 d(p3 - p2) + sum b_k (dS_k + deps),
+//   b_k = -2 w_k (p_k - F) / q_k,
+// with the rearrangements of weno5_face (weno_fast.cuh): everything in terms
+// of the second differences e_m = U_m+1 - U_m, S_k and eps four times over,
+// weights by one reciprocal of scaled products, and the three 1/q_k from one
+// more.  The gradient is formed with respect to e_1..e_4 and differenced twice
+// (e to U to W), the eps term added at the first largest |U|.  About 125
+// FP64 instructions against 220 with the three candidates and indicators
+// differentiated column by column.
+// d[0..5] = -dF/dW[0..5].
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void weno5_value_grad(const double v[5], double& D,
-                                                 double g[5]) {
-  const double a = 1.0 / 3.0, b = 7.0 / 6.0, c = 11.0 / 6.0, d = 1.0 / 6.0,
-               e = 5.0 / 6.0;
-  // eps: first maximum of v_j^2, as a chain of "if (x > m) m = x"
-  int am = 0;
-  double m = v[0] * v[0];
-#pragma unroll
-  for (int j = 1; j < 5; j++) {
-    const double s = v[j] * v[j];
-    if (s > m) { m = s; am = j; }
-  }
-  const double eps = 1e-6 * m + Consts<double>::tiny;
-  const double p1 = a * v[0] - b * v[1] + c * v[2];
-  const double p2 = -d * v[1] + e * v[2] + a * v[3];
-  const double p3 = a * v[2] + e * v[3] - d * v[4];
-  const double t1 = v[0] - 2 * v[1] + v[2], u1 = v[0] - 4 * v[1] + 3 * v[2];
-  const double t2 = v[1] - 2 * v[2] + v[3], u2 = v[1] - v[3];
-  const double t3 = v[2] - 2 * v[3] + v[4], u3 = 3 * v[2] - 4 * v[3] + v[4];
-  const double S1 = 13.0 / 12.0 * t1 * t1 + 0.25 * u1 * u1;
-  const double S2 = 13.0 / 12.0 * t2 * t2 + 0.25 * u2 * u2;
-  const double S3 = 13.0 / 12.0 * t3 * t3 + 0.25 * u3 * u3;
-  const double sc = inv_pow2_of(eps);
-  const double es = eps * sc;
-  const double q1 = S1 * sc + es, q2 = S2 * sc + es, q3 = S3 * sc + es;
-  const double Q1 = q1 * q1, Q2 = q2 * q2, Q3 = q3 * q3;
-  const double n1 = 0.1 * (Q2 * Q3), n2 = 0.6 * (Q1 * Q3), n3 = 0.3 * (Q1 * Q2);
-  const double rn = rcp_nr(n1 + n2 + n3);
-  const double w1 = n1 * rn, w2 = n2 * rn, w3 = n3 * rn;
-  D = w1 * p1 + w2 * p2 + w3 * p3;
-  const double rq = rcp_nr(q1 * q2 * q3) * sc;   // 1 / ((S1+eps)(S2+eps)(S3+eps)) / s^2
-  const double b1 = -2.0 * w1 * (p1 - D) * (q2 * q3 * rq);
-  const double b2 = -2.0 * w2 * (p2 - D) * (q1 * q3 * rq);
-  const double b3 = -2.0 * w3 * (p3 - D) * (q1 * q2 * rq);
-  const double k1 = 13.0 / 6.0 * t1, l1 = 0.5 * u1;
-  const double k2 = 13.0 / 6.0 * t2, l2 = 0.5 * u2;
-  const double k3 = 13.0 / 6.0 * t3, l3 = 0.5 * u3;
-  // dp_k and dS_k, column by column
-  g[0] = w1 * a + b1 * (k1 + l1);
-  g[1] = -w1 * b - w2 * d + b1 * (-2 * k1 - 4 * l1) + b2 * (k2 + l2);
-  g[2] = w1 * c + w2 * e + w3 * a + b1 * (k1 + 3 * l1) + b2 * (-2 * k2) +
-         b3 * (k3 + 3 * l3);
-  g[3] = w2 * a + w3 * e + b2 * (k2 - l2) + b3 * (-2 * k3 - 4 * l3);
-  g[4] = -w3 * d + b3 * (k3 + l3);
-  const double bs = (b1 + b2 + b3) * 2e-6 * v[am];
-  g[am] += bs;
+__device__ __forceinline__ void weno5_grad(const double W[6], double& F, double d[6]) {
+  const double U1 = W[1] - W[0], U2 = W[2] - W[1], U3 = W[3] - W[2], U4 = W[4] - W[3],
+               U5 = W[5] - W[4];
+  int am = 1;
+  double um = U1;
+  if (fabs(U2) > fabs(um)) { um = U2; am = 2; }
+  if (fabs(U3) > fabs(um)) { um = U3; am = 3; }
+  if (fabs(U4) > fabs(um)) { um = U4; am = 4; }
+  if (fabs(U5) > fabs(um)) { um = U5; am = 5; }
+  const double eps = fma(4e-6, um * um, 4 * Consts<double>::tiny);
+  const double e1 = U2 - U1, e2 = U3 - U2, e3 = U4 - U3, e4 = U5 - U4;
+  const double ta = e2 - e1, tb = e3 - e2, tc = e4 - e3;
+  const double ra = fma(2.0, e2, ta), rb = e2 + e3, rc = fma(-2.0, e3, tc);
+  const double ka = 13.0 / 3.0 * ta, kb = 13.0 / 3.0 * tb, kc = 13.0 / 3.0 * tc;
+  const double sc = inv_pow2_of(eps), es = mantissa_of(eps);
+  const double qa = fma(fma(ra, ra, ka * ta), sc, es), qb = fma(fma(rb, rb, kb * tb), sc, es),
+               qc = fma(fma(rc, rc, kc * tc), sc, es);
+  const double qab = qa * qb, qac = qa * qc, qbc = qb * qc;
+  const double Pab = qab * qab, Pac = qac * qac, Pbc = qbc * qbc;
+  const double rn = rcp_nr(fma(3.0, Pab, fma(6.0, Pac, Pbc)));
+  const double w1 = Pbc * rn, w2 = 6.0 * (Pac * rn), w3 = 3.0 * (Pab * rn);
+  const double h1 = 1.0 / 3.0 * (ta - tb), h3 = 1.0 / 6.0 * (tb - tc);   // p1 - p2, p3 - p2
+  const double del = fma(w1, h1, w3 * h3);                               // F - p2
+  F = fma(1.0 / 3.0, e3, fma(1.0 / 6.0, e2, U3)) + del;
+  // 2 b_k (the S_k are quadratic: dS = 2 (13/3 t dt + r dr))
+  const double rq = -4.0 * (rcp_nr(qab * qc) * sc);
+  const double b1 = w1 * (h1 - del) * (qbc * rq);
+  const double b2 = -w2 * del * (qac * rq);
+  const double b3 = w3 * (h3 - del) * (qab * rq);
+  const double Ka = b1 * ka, La = b1 * ra, Kb = b2 * kb, Lb = b2 * rb, Kc = b3 * kc,
+               Lc = b3 * rc;
+  const double v1 = 1.0 / 3.0 * w1, v3 = 1.0 / 6.0 * w3;
+  const double g1 = -(Ka + La) - v1;
+  const double g2 = (Ka + fma(3.0, La, Lb - Kb)) + fma(2.0, v1, 1.0 / 6.0 - v3);
+  const double g3 = (Kb + fma(-3.0, Lc, Lb - Kc)) + fma(2.0, v3, 1.0 / 3.0 - v1);
+  const double g4 = (Kc + Lc) - v3;
+  // deps = 8e-6 U_am dU_am; half of it, since the b are doubled
+  const double bs = (b1 + b2 + b3) * (4e-6 * um);
+  const double f1 = (am == 1 ? bs : 0.0) - g1, f2 = (am == 2 ? bs : 0.0) + (g1 - g2),
+               f3 = (am == 3 ? bs : 0.0) + ((g2 - g3) + 1.0),
+               f4 = (am == 4 ? bs : 0.0) + (g3 - g4), f5 = (am == 5 ? bs : 0.0) + g4;
+  d[0] = f1;
+  d[1] = f2 - f1;
+  d[2] = f3 - f2;
+  d[3] = f4 - f3;
+  d[4] = f5 - f4;
+  d[5] = -f5;
 }
 
 // Upwind derivative at the centre of w[0..6] = u(c-3..c+3) and its partials
-// dD/dw[0..6]; minus side when vel > 0 (v = differences of w[0..5]), plus
-// side otherwise (v = differences of w[6..1]); zero below the zero tolerance.
-__device__ __forceinline__ double upwind_grad(const double* w, double inv,
-                                              double vel, double dw[7]) {
+// times ``scale``, dw[0..6]: the minus side (w[0..5]) when vel > 0, else the
+// plus side (w[6..1], whose value is -F of the reversed stencil); zero below
+// the zero tolerance.  Both sides through one evaluation.
+__device__ __forceinline__ double upwind_grad(const double* w, double inv, double vel,
+                                              double scale, double dw[7]) {
 #pragma unroll
   for (int m = 0; m < 7; m++) dw[m] = 0.0;
   if (fabs(vel) < Consts<double>::zero_tol) return 0.0;
-  double v[5], g[5], D;
-  if (vel > 0) {
+  const bool minus = vel > 0;
+  double W[6], d[6], F;
 #pragma unroll
-    for (int j = 0; j < 5; j++) v[j] = (w[j + 1] - w[j]) * inv;
-    weno5_value_grad(v, D, g);
-    // v_j = (w_{j+1} - w_j) inv (0-based j)
+  for (int m = 0; m < 6; m++) W[m] = minus ? w[m] : w[6 - m];
+  weno5_grad(W, F, d);
+  const double si = minus ? inv : -inv;
+  const double c = -scale * si;
 #pragma unroll
-    for (int j = 0; j < 5; j++) {
-      dw[j + 1] += g[j] * inv;
-      dw[j] -= g[j] * inv;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 5; j++) v[j] = (w[6 - j] - w[5 - j]) * inv;
-    weno5_value_grad(v, D, g);
-#pragma unroll
-    for (int j = 0; j < 5; j++) {
-      dw[6 - j] += g[j] * inv;
-      dw[5 - j] -= g[j] * inv;
-    }
-  }
-  return D;
+  for (int m = 0; m < 7; m++)
+    dw[m] = c * (minus ? (m < 6 ? d[m < 6 ? m : 0] : 0.0) : (m > 0 ? d[m > 0 ? 6 - m : 0] : 0.0));
+  return F * si;
 }
 
 struct AdjParams {
@@ -148,6 +139,7 @@ struct AdjParams {
   Box gb;
   FillBox fb;             // the domain (fill box = domain box)
   double inv[3];
+  int tz;                 // planes per block (adj_tz)
 };
 
 // index of (i,j,k) in a gb array
@@ -178,26 +170,6 @@ __device__ __forceinline__ void add_target(const AdjParams& p, int i, int j, int
   atomicAdd(p.T + aix(p.gb, i, j, k), val);
 }
 
-// linear-extrapolation value of u at a point at most one axis outside
-__device__ __forceinline__ double load_bc(const AdjParams& p, int i, int j, int k) {
-  const FillBox& f = p.fb;
-  int c[3] = {i, j, k};
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    if (c[d] < f.lo[d] || c[d] > f.hi[d]) {
-      const bool lo = c[d] < f.lo[d];
-      const int dist = lo ? f.lo[d] - c[d] : c[d] - f.hi[d];
-      int e0[3] = {c[0], c[1], c[2]}, e1[3] = {c[0], c[1], c[2]};
-      e0[d] = lo ? f.lo[d] : f.hi[d];
-      e1[d] = lo ? f.lo[d] + 1 : f.hi[d] - 1;
-      const double a = __ldg(p.phi + aix(p.gb, e0[0], e0[1], e0[2]));
-      const double b = __ldg(p.phi + aix(p.gb, e1[0], e1[1], e1[2]));
-      return a + (a - b) * (double)dist;
-    }
-  }
-  return __ldg(p.phi + aix(p.gb, i, j, k));
-}
-
 // Transposed Jacobian of the upwind advection RHS.  Every cell c owns the
 // partials -V_d(c) mu(c) dD_d(c)/du(p) of its stencil points p.  The z
 // contributions go through a 7-plane register ring along the march; the x/y
@@ -205,6 +177,9 @@ __device__ __forceinline__ double load_bc(const AdjParams& p, int i, int j, int 
 // cell) and gathered by the thread of each target cell, without atomics.
 // Each finished plane of the ring and the contributions to the neighbouring
 // tiles (3-cell strips) are added to T with atomics.
+// The FP64 arithmetic and the two barriers a plane bound it; the state's
+// ghost cells are read as stored (boundary values made on the fly, and the
+// gradient by columns, took 87 us a launch at 80x72x64 where this takes 52).
 __global__ void __launch_bounds__(kTX * kTY, 2)
 k_adjoint_stage(AdjParams p) {
   __shared__ double tile[kTY + 6][kTX + 6];
@@ -213,8 +188,8 @@ k_adjoint_stage(AdjParams p) {
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i = p.fb.lo[0] + (int)blockIdx.x * kTX + tx;
   const int j = p.fb.lo[1] + (int)blockIdx.y * kTY + ty;
-  const int kb = p.fb.lo[2] + (int)blockIdx.z * kTZ;
-  const int ke = min(kb + kTZ - 1, p.fb.hi[2]);
+  const int kb = p.fb.lo[2] + (int)blockIdx.z * p.tz;
+  const int ke = min(kb + p.tz - 1, p.fb.hi[2]);
   const bool act = i <= p.fb.hi[0] && j <= p.fb.hi[1];
   const int hi0 = p.fb.hi[0], hi1 = p.fb.hi[1];
   const bool ctr_halo = !act && i <= hi0 + 3 && j <= hi1 + 3 && !(i > hi0 && j > hi1);
@@ -224,14 +199,8 @@ k_adjoint_stage(AdjParams p) {
   const bool has_hy = (i <= hi0) && ((ty < 3) || (ty >= kTY - 3 && j <= hi1));
   const int tcol = (tx < 3) ? tx : tx + 6;
   const int trow = (ty < 3) ? ty : ty + 6;
-  // tiles whose stencils stay inside the domain load without boundary tests
-  const int x0 = p.fb.lo[0] + (int)blockIdx.x * kTX, y0 = p.fb.lo[1] + (int)blockIdx.y * kTY;
-  const bool inside = x0 - 3 >= p.fb.lo[0] && min(x0 + kTX - 1, hi0) + 3 <= hi0 &&
-                      y0 - 3 >= p.fb.lo[1] && min(y0 + kTY - 1, hi1) + 3 <= hi1 &&
-                      kb - 3 >= p.fb.lo[2] && ke + 3 <= p.fb.hi[2];
-  auto ld = [&](int a, int b, int c) -> double {
-    return inside ? __ldg(p.phi + aix(p.gb, a, b, c)) : load_bc(p, a, b, c);
-  };
+  // the ghost cells of the state hold its boundary values
+  auto ld = [&](int a, int b, int c) -> double { return __ldg(p.phi + aix(p.gb, a, b, c)); };
 
   // registers of the next plane (loaded while the current one is worked):
   // the new top of the z window or the own cell (halo threads), the strip
@@ -294,11 +263,10 @@ k_adjoint_stage(AdjParams p) {
         double wx[7], d7[7];
 #pragma unroll
         for (int m = 0; m < 7; m++) wx[m] = tile[ty + 3][tx + m];
-        Dx = upwind_grad(wx, p.inv[0], vx, d7);
-        const double sx = -vx * mu;
+        Dx = upwind_grad(wx, p.inv[0], vx, -vx * mu, d7);
 #pragma unroll
         for (int m = 0; m < 7; m++) {
-          double c = sx * d7[m];
+          double c = d7[m];
           const int ti = i + m - 3;
           if (ti < p.fb.lo[0] || ti > hi0) {
             if (c != 0.0) add_target(p, ti, j, k, c);
@@ -311,11 +279,10 @@ k_adjoint_stage(AdjParams p) {
         double wy[7], d7[7];
 #pragma unroll
         for (int m = 0; m < 7; m++) wy[m] = tile[ty + m][tx + 3];
-        Dy = upwind_grad(wy, p.inv[1], vy, d7);
-        const double sy = -vy * mu;
+        Dy = upwind_grad(wy, p.inv[1], vy, -vy * mu, d7);
 #pragma unroll
         for (int m = 0; m < 7; m++) {
-          double c = sy * d7[m];
+          double c = d7[m];
           const int tj = j + m - 3;
           if (tj < p.fb.lo[1] || tj > hi1) {
             if (c != 0.0) add_target(p, i, tj, k, c);
@@ -326,10 +293,9 @@ k_adjoint_stage(AdjParams p) {
       }
       {
         double d7[7];
-        Dz = upwind_grad(w, p.inv[2], vz, d7);
-        const double sz = -vz * mu;
+        Dz = upwind_grad(w, p.inv[2], vz, -vz * mu, d7);
 #pragma unroll
-        for (int m = 0; m < 7; m++) ring[m] += sz * d7[m];   // ring[m]: plane k+m-3
+        for (int m = 0; m < 7; m++) ring[m] += d7[m];   // ring[m]: plane k+m-3
       }
       p.A[0][o] = a0 - mu * Dx;
       p.A[1][o] = a1 - mu * Dy;
@@ -621,6 +587,18 @@ cudaError_t fwd_step(lsmgpu_adjoint* h, double* out, const double* in, cudaStrea
   return fwd_stage(h, out, h->s2, in, 33, st);
 }
 
+// Planes per block of k_adjoint_stage: at most 8, and few enough for two
+// waves of blocks (two per SM).  Reverse sweep of 24 steps at 80x72x64: 6.1 ms
+// with 16 planes (108 blocks), 4.2 with 8, 3.7 with 3 (594); of 20 steps at
+// 40x30x35 4.5, 2.6 and 1.2 (2 planes); of 48 steps at 128^3 30.8 with 6 to
+// 16, 33.2 with 2.
+int adj_tz(const FillBox& fb) {
+  const long tiles = (long)((fb.n(0) + kTX - 1) / kTX) * ((fb.n(1) + kTY - 1) / kTY);
+  int tz = 8;
+  while (tz > 1 && tiles * ((fb.n(2) + tz - 1) / tz) < 2 * 2 * 148) tz--;
+  return tz;
+}
+
 // T += J(u)^T mu with mu = coef (ca sa + cb sb); T must be zero on entry, sb
 // (a consumed accumulation buffer, or null) is zeroed as it is read
 cudaError_t adj_kernel(lsmgpu_adjoint* h, const double* u, const double* sa, double ca,
@@ -638,8 +616,9 @@ cudaError_t adj_kernel(lsmgpu_adjoint* h, const double* u, const double* sa, dou
   p.T = T;
   p.gb = h->gb;
   p.fb = h->fb;
+  p.tz = adj_tz(h->fb);
   dim3 grid((h->fb.n(0) + kTX - 1) / kTX, (h->fb.n(1) + kTY - 1) / kTY,
-            (h->fb.n(2) + kTZ - 1) / kTZ);
+            (h->fb.n(2) + p.tz - 1) / p.tz);
   k_adjoint_stage<<<grid, dim3(kTX, kTY), 0, st>>>(p);
   ++launch_counter();
   return cudaGetLastError();
@@ -656,7 +635,15 @@ cudaError_t recompute_segment(lsmgpu_adjoint* h, int c, int b, cudaStream_t st) 
     const double* u = q == 0 ? h->ckpt[c] : set[0][q];
     if ((e = fwd_stage(h, set[1][q], u, u, 1, st))) return e;
     if ((e = fwd_stage(h, set[2][q], set[1][q], u, 32, st))) return e;
-    if (s + 1 < s1 && (e = fwd_stage(h, set[0][q + 1], set[2][q], u, 33, st))) return e;
+    // (the reverse sweep reads the ghost cells of every state; a state's first
+    // stage or this fills them)
+    if (s + 1 < s1) {
+      if ((e = fwd_stage(h, set[0][q + 1], set[2][q], u, 33, st))) return e;
+    } else {
+      StageArgs a = fwd_args(h);
+      a.phi_s = set[2][q];
+      if ((e = launch_ghosts(8, a, st))) return e;
+    }
   }
   return cudaSuccess;
 }

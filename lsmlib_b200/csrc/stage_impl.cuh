@@ -195,6 +195,12 @@ cudaError_t band_kind(dim3 grid, const StageArgs& a32, const StageArgs& a64,
 }  // namespace
 
 #ifdef STAGE_BAND_FN
+cudaError_t launch_ghosts(int prec, const StageArgs& a, cudaStream_t st) {
+  if (prec == 8) launch_face_ghosts<double>(a, st);
+  else launch_face_ghosts<float>(a, st);
+  return cudaGetLastError();
+}
+
 cudaError_t STAGE_BAND_FN(int kind, const StageArgs& a32, const StageArgs& a64,
                           const unsigned char* tile_fp64, cudaStream_t st, cudaStream_t side,
                           cudaEvent_t ev[2]) {

@@ -92,6 +92,9 @@ cudaError_t launch_stage_strict(int kind, int prec, const StageArgs& a,
                                 cudaStream_t st);
 cudaError_t launch_stage_fast(int kind, int prec, const StageArgs& a,
                               cudaStream_t st);
+// The boundary values of a.bc_mask into the face ghost cells of a.phi_s that
+// the stencils of a.fb reach (at least 3 domain cells per axis).
+cudaError_t launch_ghosts(int prec, const StageArgs& a, cudaStream_t st);
 // One stage of kStageDeformation (velocity evaluated in the kernel, so both
 // precisions have it) in the FP64 band form, fast arithmetic: a32 and a64 name the same stage over the FP32
 // arrays and their FP64 copies; tile_fp64[tile] (tiles as in stage_blocks,
