@@ -888,7 +888,7 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
         float2 a[6], vp, vm;
 #pragma unroll
         for (int m = 0; m < 6; m++) a[m] = make_float2(u[m], u[m + 1]);
-        weno5_face2(a, p.inv[0], vp, vm);
+        weno5_face2<true>(a, p.inv[0], vp, vm);
         xp0 = vp.x; xp1 = vp.y; xm1 = vm.x; xnext = vm.y;
 #pragma unroll
         for (int m = 0; m < 6; m++) a[m] = make_float2(ya[m], yb[m]);
@@ -1207,16 +1207,21 @@ k_stage(StageParams<T> p) {
   block_max_partial<KIND, TX * TY>(p, hmax);
 }
 
-// blocks per SM the register allocation of the pair kernel must allow
-#ifndef LSMGPU_PAIR_MIN_BLOCKS
-#define LSMGPU_PAIR_MIN_BLOCKS 4
-#endif
+// Blocks per SM the register allocation of a pair kernel must allow.  FP64: 4
+// (128 registers; 5 spill, reinitialization at 257^3 499 us against 404).
+// FP32 without the FP64 kinks fits 96 registers, and 80 for the velocity
+// arrays, and gains from the warps: with 4 blocks reinitialization 276 us,
+// normal speed 279, velocity arrays 289, deformation 276 at 257^3, so 258, 271,
+// 246 and 263.  The FP64 band form shares the SMs between both precisions'
+// launches and keeps 4 (10 steps at 192x176x160 4.48 ms, 4.56 with 5).
+template <typename T, int KIND, bool K64, bool BAND = false>
+constexpr int kPairBlocks = sizeof(T) == 8 || K64 || BAND ? 4 : KIND == kStageAdvect ? 6 : 5;
 
 // The face-shared two-sided kinds, two cells per thread (stage_tile_pairs):
 // a block of kPairThreads threads covers the same 32 x 8 x tz tile as k_stage.
 // Every ghost cell the stencils reach is read as stored.
 template <typename T, int KIND, bool K64>
-__global__ void __launch_bounds__(kPairThreads, LSMGPU_PAIR_MIN_BLOCKS)
+__global__ void __launch_bounds__(kPairThreads, (kPairBlocks<T, KIND, K64>))
 k_stage_pairs(StageParams<T> p) {
   __shared__ __align__(16) T tile[2][kPairRows][kPairTX + 8];
   __shared__ __align__(16) T fy[2 * kPairThreads + kPairTX];
@@ -1231,7 +1236,7 @@ k_stage_pairs(StageParams<T> p) {
 // (the tiles whose tile_fp64 flag is tile_want, out_alt written as well; the
 // flags number 32 x 8 x kStageTZ tiles, so its columns are never narrow).
 template <typename T, int KIND, bool K64, bool BAND = false>
-__global__ void __launch_bounds__(kPairThreads, LSMGPU_PAIR_MIN_BLOCKS)
+__global__ void __launch_bounds__(kPairThreads, (kPairBlocks<T, KIND, K64, BAND>))
 k_stage_pairs_up(StageParams<T> p) {
   __shared__ __align__(16) T tile[2][BAND ? kPairTY + 6 : kPairRows][kPairTX + 8];
   if constexpr (BAND) {

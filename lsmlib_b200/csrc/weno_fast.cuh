@@ -346,40 +346,41 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 // a - b, rounded once (b * -1 is exact)
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.0f), a); }
 
+// XPAIR: lane y is the face one cell on from lane x (u[m].y = u[m+1].x), so
+// the maximum of the four common |V| is taken once.
+template <bool XPAIR = false>
 __device__ __forceinline__ void weno5_face2(const float2* u, float inv, float2& vp, float2& vm) {
   const float2 V1 = sub2(u[1], u[0]), V2 = sub2(u[2], u[1]), V3 = sub2(u[3], u[2]),
                V4 = sub2(u[4], u[3]), V5 = sub2(u[5], u[4]);
   float2 amax;
-  amax.x = vmax(vmax(vmax(fabsf(V1.x), fabsf(V2.x)), vmax(fabsf(V3.x), fabsf(V4.x))), fabsf(V5.x));
-  amax.y = vmax(vmax(vmax(fabsf(V1.y), fabsf(V2.y)), vmax(fabsf(V3.y), fabsf(V4.y))), fabsf(V5.y));
-  const float2 m = mul2(amax, amax);
-  // S_k and eps four times over, as in weno5_face
-  const float2 eps = fma2(f2(4e-6f), m, f2(4.0f * Consts<float>::tiny));
+  if (XPAIR) {
+    const float m = vmax(vmax(fabsf(V2.x), fabsf(V3.x)), vmax(fabsf(V4.x), fabsf(V5.x)));
+    amax = make_float2(vmax(fabsf(V1.x), m), vmax(m, fabsf(V5.y)));
+  } else {
+    amax.x = vmax(vmax(vmax(fabsf(V1.x), fabsf(V2.x)), vmax(fabsf(V3.x), fabsf(V4.x))), fabsf(V5.x));
+    amax.y = vmax(vmax(vmax(fabsf(V1.y), fabsf(V2.y)), vmax(fabsf(V3.y), fabsf(V4.y))), fabsf(V5.y));
+  }
+  const float2 eps = fma2(f2(4e-6f), mul2(amax, amax), f2(4.0f * Consts<float>::tiny));
   const float2 c13_3 = f2(13.0f / 3.0f);
-  const float2 ta = add2(fma2(f2(-2.0f), V2, V1), V3);
-  const float2 tb = add2(fma2(f2(-2.0f), V3, V2), V4);
-  const float2 tc = add2(fma2(f2(-2.0f), V4, V3), V5);
-  float2 t = fma2(f2(3.0f), V3, fma2(f2(-4.0f), V2, V1));
-  const float2 Sa = fma2(mul2(c13_3, ta), ta, mul2(t, t));
-  t = sub2(V2, V4);
-  const float2 Sb = fma2(mul2(c13_3, tb), tb, mul2(t, t));
-  t = add2(fma2(f2(-4.0f), V4, mul2(f2(3.0f), V3)), V5);
-  const float2 Sc = fma2(mul2(c13_3, tc), tc, mul2(t, t));
+  const float2 e1 = sub2(V2, V1), e2 = sub2(V3, V2), e3 = sub2(V4, V3), e4 = sub2(V5, V4);
+  const float2 ta = sub2(e2, e1), tb = sub2(e3, e2), tc = sub2(e4, e3);
+  const float2 ra = fma2(f2(2.0f), e2, ta), rb = add2(e2, e3), rc = fma2(f2(-2.0f), e3, tc);
+  const float2 Sa = fma2(ra, ra, mul2(mul2(c13_3, ta), ta));
+  const float2 Sb = fma2(rb, rb, mul2(mul2(c13_3, tb), tb));
+  const float2 Sc = fma2(rc, rc, mul2(mul2(c13_3, tc), tc));
   const float2 sc = make_float2(inv_pow2_of(eps.x), inv_pow2_of(eps.y));
   const float2 es = mul2(eps, sc);
   const float2 qa = fma2(Sa, sc, es), qb = fma2(Sb, sc, es), qc = fma2(Sc, sc, es);
   const float2 Qa = mul2(qa, qa), Qb = mul2(qb, qb), Qc = mul2(qc, qc);
   const float2 Pbc = mul2(Qb, Qc), Pac = mul2(Qa, Qc), Pab = mul2(Qa, Qb);
   const float2 A = mul2(Pbc, sub2(ta, tb)), B = mul2(Pab, sub2(tb, tc));
-  // halved numerators and weight sums, as in weno5_face
   const float2 num_m = fma2(f2(1.5f), B, A);
-  const float2 num_p = fma2(f2(1.5f), A, B);
-  const float2 e3 = mul2(f2(5.0f / 6.0f), V3);
-  const float2 p2m = fma2(f2(1.0f / 3.0f), V4, fma2(f2(-1.0f / 6.0f), V2, e3));
-  const float2 p2p = fma2(f2(1.0f / 3.0f), V2, fma2(f2(-1.0f / 6.0f), V4, e3));
-  const float2 p18 = mul2(f2(18.0f), Pac);
-  const float2 sm = fma2(f2(3.0f), Pbc, fma2(f2(9.0f), Pab, p18));
-  const float2 sp = fma2(f2(3.0f), Pab, fma2(f2(9.0f), Pbc, p18));
+  const float2 num_p = fma2(f2(-1.5f), A, mul2(f2(-1.0f), B));   // negated
+  // three times the middle candidates
+  const float2 p2m = fma2(f2(3.0f), V3, fma2(f2(0.5f), e2, e3));
+  const float2 p2p = fma2(f2(-1.5f), rb, p2m);
+  const float2 sm = fma2(f2(3.0f), Pab, fma2(f2(6.0f), Pac, Pbc));
+  const float2 sp = fma2(f2(3.0f), Pbc, fma2(f2(6.0f), Pac, Pab));
   // reciprocals: per-lane seeds, one packed Newton-Raphson step (rcp_nr)
   float2 rm, rp;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rm.x) : "f"(sm.x));
@@ -388,8 +389,9 @@ __device__ __forceinline__ void weno5_face2(const float2* u, float inv, float2& 
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rp.y) : "f"(sp.y));
   rm = fma2(rm, fma2(mul2(f2(-1.0f), sm), rm, f2(1.0f)), rm);
   rp = fma2(rp, fma2(mul2(f2(-1.0f), sp), rp, f2(1.0f)), rp);
-  vm = mul2(fma2(num_m, rm, p2m), f2(inv));
-  vp = mul2(fma2(mul2(f2(-1.0f), num_p), rp, p2p), f2(inv));
+  const float2 i3 = f2(inv * (1.0f / 3.0f));
+  vm = mul2(fma2(num_m, rm, p2m), i3);
+  vp = mul2(fma2(num_p, rp, p2p), i3);
 }
 
 // weno5_side_fast<float> for two independent sides at once, one per lane of
