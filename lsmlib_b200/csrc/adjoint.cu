@@ -182,6 +182,7 @@ __device__ __forceinline__ void add_target(const AdjParams& p, int i, int j, int
 // gradient by columns, took 87 us a launch at 80x72x64 where this takes 52).
 __global__ void __launch_bounds__(kTX * kTY, 2)
 k_adjoint_stage(AdjParams p) {
+  grid_wait();
   __shared__ double tile[kTY + 6][kTX + 6];
   __shared__ double Cx[7][kTY][kTX];
   __shared__ double Cy[7][kTY][kTX];
@@ -359,6 +360,7 @@ k_adjoint_stage(AdjParams p) {
 // consumed (zeroed for the next step's accumulation)
 __global__ void k_adj_combine(double* out, const double* lam, const double* lam2,
                               const double* lam1, double* T1, Box gb, FillBox fb) {
+  grid_wait();
   const int i = fb.lo[0] + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = fb.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
   if (i > fb.hi[0] || j > fb.hi[1]) return;
@@ -619,7 +621,14 @@ cudaError_t adj_kernel(lsmgpu_adjoint* h, const double* u, const double* sa, dou
   p.tz = adj_tz(h->fb);
   dim3 grid((h->fb.n(0) + kTX - 1) / kTX, (h->fb.n(1) + kTY - 1) / kTY,
             (h->fb.n(2) + p.tz - 1) / p.tz);
-  k_adjoint_stage<<<grid, dim3(kTX, kTY), 0, st>>>(p);
+  // Beyond three waves a successor that waits on the SMs costs the recomputation
+  // beside it more than the gap (reverse sweep at 128^3, 1,024 blocks: 29.3 ms
+  // against 28.2); below, 3.49 against 3.61 at 80x72x64 and 0.88 against 1.03
+  // at 40x30x35.
+  if (grid.x * grid.y * grid.z <= 3 * 2 * 148)
+    launch_after(k_adjoint_stage, grid, dim3(kTX, kTY), st, p);
+  else
+    k_adjoint_stage<<<grid, dim3(kTX, kTY), 0, st>>>(p);
   ++launch_counter();
   return cudaGetLastError();
 }
@@ -666,9 +675,11 @@ cudaError_t adj_step(lsmgpu_adjoint* h, const double* u, const double* s1,
   // T <- J(u)^T mu1
   if ((e = adj_kernel(h, u, h->lam2, 0.25, h->Tb, 1.0, dt, h->lam1, h->T, st))) return e;
   // lam <- 1/3 lam + 3/4 lam2 + lam1 + T1 (T consumed)
-  dim3 blk(32, 4, 1), grid((h->fb.n(0) + 31) / 32, (h->fb.n(1) + 3) / 4,
-                           h->fb.n(2) < 65535 ? h->fb.n(2) : 65535);
-  k_adj_combine<<<grid, blk, 0, st>>>(h->lam, h->lam, h->lam2, h->lam1, h->T, h->gb, h->fb);
+  // (blocks loop over planes: see launch_rk)
+  const int zb = h->fb.n(2) < 32 ? h->fb.n(2) : 32;
+  dim3 blk(32, 4, 1), grid((h->fb.n(0) + 31) / 32, (h->fb.n(1) + 3) / 4, zb);
+  launch_after(k_adj_combine, grid, blk, st, h->lam, h->lam, h->lam2, h->lam1, h->T, h->gb,
+               h->fb);
   ++launch_counter();
   return cudaGetLastError();
 }

@@ -115,6 +115,37 @@ __device__ __forceinline__ float sr_float(double x, unsigned r) {
   return (float)__longlong_as_double((long long)(mag | sign));
 }
 
+// Programmatic dependent launch of the drivers' chains of short kernels: a
+// kernel launched with launch_after may become resident while the kernel
+// before it still runs, and waits here until that one has completed and its
+// writes are visible; only then may it touch memory.  Every thread of every
+// block calls it first (a grid that ended without waiting would let its
+// successor overtake the grid before it).  It also lets the next kernel of
+// the chain become resident.  No effect in a kernel launched normally.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+}
+
+// Launch ``kernel`` (which begins with grid_wait) behind the work on st without
+// the gap between two kernels: 1.5 to 2 us a launch.  Reinitialization stage
+// with its ghost fill, FP64: 33^3 12.3 -> 8.9 us, 65^3 20.6 -> 17.8,
+// 130x98x132 57.4 -> 54.5, 257^3 403.6 -> 400.8.
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st,
+                                A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Status word that kernels may raise (never trap): bit 0 = bad argument seen
 // on the device, bit 1 = a bounded wait gave up.
 enum DeviceStatus : unsigned { kDevOk = 0u, kDevBadArg = 1u, kDevTimeout = 2u };

@@ -95,10 +95,17 @@ enum { kDt = 0, kT = 1, kDtLast = 2, kG0 = 3, kNumScal = 8 };
 
 __device__ __forceinline__ double gmax(double m, double v) { return v > m ? v : m; }
 
+// The step's end, as soon as nothing of the step reads t any more
+__device__ __forceinline__ void advance_t(double* scal) {
+  scal[kT] = scal[kT] + scal[kDt];
+  scal[kDtLast] = scal[kDt];
+}
+
 // dt = cfl / (max + tiny) (lsm_utilities3d.f.in:322, :445), optionally
-// clipped so that t + dt does not pass t_end
+// clipped so that t + dt does not pass t_end; ``advance``: the step's end too
 __global__ void k_dt_finish(const double* partials, int np, double cfl,
-                            double tiny, double* scal, double t_end) {
+                            double tiny, double* scal, double t_end, int advance) {
+  grid_wait();
   __shared__ double red[8];
   double m = -1.0;
   for (int t = threadIdx.x; t < np; t += blockDim.x) m = gmax(m, partials[t]);
@@ -111,13 +118,14 @@ __global__ void k_dt_finish(const double* partials, int np, double cfl,
     double dt = cfl / (m + tiny);
     if (t_end > 0.0 && scal[kT] + dt > t_end) dt = t_end - scal[kT];
     scal[kDt] = dt;
+    if (advance) advance_t(scal);
   }
 }
 
-__global__ void k_set_dt(double* scal, double dt) { scal[kDt] = dt; }
-__global__ void k_advance_t(double* scal) {
-  scal[kT] = scal[kT] + scal[kDt];
-  scal[kDtLast] = scal[kDt];
+__global__ void k_set_dt(double* scal, double dt) {
+  grid_wait();
+  scal[kDt] = dt;
+  advance_t(scal);
 }
 
 // LeVeque's 3D deformation field (deformation_velocity, stage.cuh) at cell
@@ -129,6 +137,7 @@ __global__ void k_advance_t(double* scal) {
 // tabulation.
 __global__ void k_deform_tables(double* tab, FillBox fb, double x0, double y0,
                                 double z0, double dx, double dy, double dz) {
+  grid_wait();
   const int n0 = fb.n(0), n1 = fb.n(1), n2 = fb.n(2);
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   double x;
@@ -153,10 +162,14 @@ __device__ __forceinline__ double deform_g(const double* scal, double c, double 
   return cos(M_PI * t / period);
 }
 
-// g at the three stage times t, t + dt, t + dt/2 (after this step's dt)
+// g at the three stage times t, t + dt, t + dt/2 (after this step's dt), and
+// the step's end (one warp)
 __global__ void k_deform_g(double* scal, double period) {
+  grid_wait();
   const double c[3] = {0.0, 1.0, 0.5};
   if (threadIdx.x < 3) scal[kG0 + threadIdx.x] = deform_g(scal, c[threadIdx.x], period);
+  __syncwarp();
+  if (threadIdx.x == 0) advance_t(scal);
 }
 
 // the CFL reduction of the deformation field at time t (FP64), over the
@@ -166,6 +179,7 @@ template <typename T>
 __global__ void k_deform_partials(const double* tab, FillBox fb, const double* scal,
                                   double period, double ix, double iy, double iz,
                                   double* partials) {
+  grid_wait();
   const double g = deform_g(scal, 0.0, period);
   const int n0 = fb.n(0), n1 = fb.n(1), n2 = fb.n(2);
   double m = -1.0;
@@ -199,6 +213,7 @@ template <typename T>
 __global__ void k_adv_partials(const T* vx, const T* vy, const T* vz, Box gb,
                                FillBox fb, double ix, double iy, double iz,
                                double* partials) {
+  grid_wait();
   double m = -1.0;
   const long n = fb.count();
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n;
@@ -781,20 +796,20 @@ int lsmgpu_advect_tvdrk3(lsmgpu_workspace* ws, void* phi, const void* vx,
   const double tiny = ws->prec == 8 ? Consts<double>::tiny : (double)Consts<float>::tiny;
   for (int s = 0; s < nsteps; s++) {
     if (dt_fixed > 0) {
-      k_set_dt<<<1, 1, 0, st>>>(ws->scal, dt_fixed);
+      launch_after(k_set_dt, 1, 1, st, ws->scal, dt_fixed);
     } else {
       const double inv[3] = {1.0 / dx[0], 1.0 / dx[1], 1.0 / dx[2]};
       if (ws->prec == 8)
-        k_adv_partials<double><<<kAdvRedBlocks, 256, 0, st>>>(
-            (const double*)vx, (const double*)vy, (const double*)vz, ws->gb, f,
-            inv[0], inv[1], inv[2], ws->partials);
+        launch_after(k_adv_partials<double>, kAdvRedBlocks, 256, st, (const double*)vx,
+                     (const double*)vy, (const double*)vz, ws->gb, f, inv[0], inv[1], inv[2],
+                     ws->partials);
       else
-        k_adv_partials<float><<<kAdvRedBlocks, 256, 0, st>>>(
-            (const float*)vx, (const float*)vy, (const float*)vz, ws->gb, f,
-            inv[0], inv[1], inv[2], ws->partials);
+        launch_after(k_adv_partials<float>, kAdvRedBlocks, 256, st, (const float*)vx,
+                     (const float*)vy, (const float*)vz, ws->gb, f, inv[0], inv[1], inv[2],
+                     ws->partials);
       ++launch_counter();
-      k_dt_finish<<<1, 256, 0, st>>>(ws->partials, kAdvRedBlocks, cfl, tiny,
-                                     ws->scal, t_end);
+      launch_after(k_dt_finish, 1, 256, st, ws->partials, kAdvRedBlocks, cfl, tiny, ws->scal,
+                   t_end, 1);
     }
     ++launch_counter();
     StageArgs a = base_args(ws, f, dx);
@@ -805,8 +820,6 @@ int lsmgpu_advect_tvdrk3(lsmgpu_workspace* ws, void* phi, const void* vx,
     if (!cuda_ok(stage(kStageAdvect, ws->prec, a, st, ws), R)) return LSMGPU_ERR_CUDA;
     a.out = phi; a.phi_s = ws->phi2; a.rk_kind = 33;
     if (!cuda_ok(stage(kStageAdvect, ws->prec, a, st, ws), R)) return LSMGPU_ERR_CUDA;
-    k_advance_t<<<1, 1, 0, st>>>(ws->scal);
-    ++launch_counter();
     ws->steps++;
   }
   if (!cuda_ok(cudaGetLastError(), R)) return LSMGPU_ERR_CUDA;
@@ -840,8 +853,8 @@ int lsmgpu_deformation_tvdrk3(lsmgpu_workspace* ws, void* phi, const int fb[6],
   }
   cudaStream_t st = cur_stream();
   const int nt = f.n(0) + f.n(1) + f.n(2);
-  k_deform_tables<<<(nt + 127) / 128, 128, 0, st>>>(ws->defo_tab, f, x_lo[0], x_lo[1],
-                                                    x_lo[2], dx[0], dx[1], dx[2]);
+  launch_after(k_deform_tables, (nt + 127) / 128, 128, st, ws->defo_tab, f, x_lo[0], x_lo[1],
+               x_lo[2], dx[0], dx[1], dx[2]);
   ++launch_counter();
   // FP64 band form: the tiles near the interface in FP64, with the dt of the
   // FP64 velocity, as an FP64 workspace computes them
@@ -858,14 +871,14 @@ int lsmgpu_deformation_tvdrk3(lsmgpu_workspace* ws, void* phi, const int fb[6],
   for (int s = 0; s < nsteps; s++) {
     // dt from the field at t (the stage-1 field)
     if (ws->prec == 8 || band)
-      k_deform_partials<double><<<kAdvRedBlocks, 256, 0, st>>>(
-          ws->defo_tab, f, ws->scal, period, inv[0], inv[1], inv[2], ws->partials);
+      launch_after(k_deform_partials<double>, kAdvRedBlocks, 256, st, ws->defo_tab, f, ws->scal,
+                   period, inv[0], inv[1], inv[2], ws->partials);
     else
-      k_deform_partials<float><<<kAdvRedBlocks, 256, 0, st>>>(
-          ws->defo_tab, f, ws->scal, period, inv[0], inv[1], inv[2], ws->partials);
-    k_dt_finish<<<1, 256, 0, st>>>(ws->partials, kAdvRedBlocks, cfl, tiny, ws->scal,
-                                   t_end);
-    k_deform_g<<<1, 32, 0, st>>>(ws->scal, period);
+      launch_after(k_deform_partials<float>, kAdvRedBlocks, 256, st, ws->defo_tab, f, ws->scal,
+                   period, inv[0], inv[1], inv[2], ws->partials);
+    launch_after(k_dt_finish, 1, 256, st, ws->partials, kAdvRedBlocks, cfl, tiny, ws->scal,
+                 t_end, 0);
+    launch_after(k_deform_g, 1, 32, st, ws->scal, period);
     launch_counter() += 3;
     StageArgs a = base_args(ws, f, dx);
     a.defo_tab = ws->defo_tab;
@@ -883,8 +896,6 @@ int lsmgpu_deformation_tvdrk3(lsmgpu_workspace* ws, void* phi, const int fb[6],
     a.g_dev = ws->scal + kG0 + 2;
     a.out = phi; a.phi_s = ws->phi2; a.rk_kind = 33;
     if (!cuda_ok(run(a), R)) return LSMGPU_ERR_CUDA;
-    k_advance_t<<<1, 1, 0, st>>>(ws->scal);
-    ++launch_counter();
     ws->steps++;
   }
   if (!cuda_ok(cudaGetLastError(), R)) return LSMGPU_ERR_CUDA;
@@ -916,7 +927,7 @@ int lsmgpu_normal_tvdrk3(lsmgpu_workspace* ws, void* phi, const void* F,
     // WENO5 +- of phi^n once: L(phi^n) for stage 1 and the CFL maxima
     a.rhs_out = ws->rhs; a.partials = ws->partials; a.phi_s = phi;
     if (!cuda_ok(stage(kStageNormalRhs, ws->prec, a, st, ws), R)) return LSMGPU_ERR_CUDA;
-    k_dt_finish<<<1, 256, 0, st>>>(ws->partials, nblk, cfl, tiny, ws->scal, 0.0);
+    launch_after(k_dt_finish, 1, 256, st, ws->partials, nblk, cfl, tiny, ws->scal, 0.0, 1);
     ++launch_counter();
     // stage 1: phi1 = phi + dt L (LSM3D_TVD_RK3_STAGE1)
     if (!cuda_ok(launch_rk(ws->prec, 1, ws->phi1, ws->gb, nullptr, ws->gb, phi,
@@ -928,8 +939,6 @@ int lsmgpu_normal_tvdrk3(lsmgpu_workspace* ws, void* phi, const void* F,
     if (!cuda_ok(stage(kStageNormal, ws->prec, a, st, ws), R)) return LSMGPU_ERR_CUDA;
     a.out = phi; a.phi_s = ws->phi2; a.rk_kind = 33;
     if (!cuda_ok(stage(kStageNormal, ws->prec, a, st, ws), R)) return LSMGPU_ERR_CUDA;
-    k_advance_t<<<1, 1, 0, st>>>(ws->scal);
-    ++launch_counter();
     ws->steps++;
     if (reinit_interval > 0 && (step0 + s + 1) % reinit_interval == 0)
       if (!reinit_run(ws, phi, f, dx, cfl, reinit_iters, use_phi0_for_sgn, st, R))
@@ -1084,7 +1093,7 @@ int lsmgpu_normal_tvdrk3_host(lsmgpu_workspace* ws, void* phi, const void* F,
       a.partials = ws->partials;
       if (!cuda_ok(stage(kStageNormalRhs, ws->prec, a, st, ws), R)) return LSMGPU_ERR_CUDA;
     }
-    k_dt_finish<<<1, 256, 0, st>>>(ws->partials, nblk, cfl, tiny, ws->scal, 0.0);
+    launch_after(k_dt_finish, 1, 256, st, ws->partials, nblk, cfl, tiny, ws->scal, 0.0, 1);
     ++launch_counter();
     if (!cuda_ok(launch_rk(ws->prec, 1, ws->phi1, ws->gb, nullptr, ws->gb, dphi, ws->gb,
                            ws->rhs, ws->gb, f, 0.0, ws->scal + kDt, st, next_sr_seed(ws)),
@@ -1112,8 +1121,6 @@ int lsmgpu_normal_tvdrk3_host(lsmgpu_workspace* ws, void* phi, const void* F,
     } else if (!cuda_ok(stage(kStageNormal, ws->prec, a, st, ws), R)) {
       return LSMGPU_ERR_CUDA;
     }
-    k_advance_t<<<1, 1, 0, st>>>(ws->scal);
-    ++launch_counter();
     ws->steps++;
     if (reinit_now && !reinit_run(ws, dphi, f, dx, cfl, reinit_iters, use_phi0_for_sgn, st, R))
       return lsmgpu_peek_last_error();

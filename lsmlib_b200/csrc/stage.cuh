@@ -1193,6 +1193,7 @@ __device__ __forceinline__ void block_max_partial(const P& p, double hmax) {
 template <typename T, int KIND, bool FAST, int TX, int TY>
 __global__ void __launch_bounds__(TX * TY, LSMGPU_STAGE_MIN_BLOCKS)
 k_stage(StageParams<T> p) {
+  grid_wait();
   __shared__ T tile[2][TY + 6][TX + 6];
   double hmax;
   if constexpr (UseFaces<T, KIND, FAST, TX>::value) {
@@ -1223,6 +1224,7 @@ constexpr int kPairBlocks = sizeof(T) == 8 || K64 || BAND ? 4 : KIND == kStageAd
 template <typename T, int KIND, bool K64>
 __global__ void __launch_bounds__(kPairThreads, (kPairBlocks<T, KIND, K64>))
 k_stage_pairs(StageParams<T> p) {
+  grid_wait();
   __shared__ __align__(16) T tile[2][kPairRows][kPairTX + 8];
   __shared__ __align__(16) T fy[2 * kPairThreads + kPairTX];
   __shared__ T fx[kPairThreads / 4];
@@ -1238,6 +1240,7 @@ k_stage_pairs(StageParams<T> p) {
 template <typename T, int KIND, bool K64, bool BAND = false>
 __global__ void __launch_bounds__(kPairThreads, (kPairBlocks<T, KIND, K64, BAND>))
 k_stage_pairs_up(StageParams<T> p) {
+  grid_wait();
   __shared__ __align__(16) T tile[2][BAND ? kPairTY + 6 : kPairRows][kPairTX + 8];
   if constexpr (BAND) {
     if (p.tile_fp64[blockIdx.x + gridDim.x * (blockIdx.y + (size_t)gridDim.y * blockIdx.z)] !=
@@ -1316,6 +1319,7 @@ __host__ __device__ inline int face_ghost_xy_blocks(int nx, int ny, int* bx = nu
 template <typename T>
 __global__ void __launch_bounds__(kFaceGhostThreads)
 k_face_ghosts(T* phi, Box gb, FillBox dom, unsigned m, int k0, int k1, int zchunks) {
+  grid_wait();
   const int nx = dom.n(0), ny = dom.n(1);
   const int ngroups = (k1 - k0 + kGhostPlanes) / kGhostPlanes;
   int bx;

@@ -70,8 +70,8 @@ void launch_face_ghosts(const StageArgs& a, cudaStream_t st) {
                 (4 * kFaceGhostThreads));
   const long groups = (a.fb.n(2) + kGhostPlanes - 1) / kGhostPlanes;
   const long blocks = groups * face_ghost_xy_blocks(a.dom.n(0), a.dom.n(1)) + 6L * zchunks;
-  k_face_ghosts<T><<<(unsigned)blocks, kFaceGhostThreads, 0, st>>>(
-      (T*)a.phi_s, a.gb, a.dom, a.bc_mask, a.fb.lo[2], a.fb.hi[2], zchunks);
+  launch_after(k_face_ghosts<T>, (unsigned)blocks, kFaceGhostThreads, st, (T*)a.phi_s, a.gb,
+               a.dom, a.bc_mask, a.fb.lo[2], a.fb.hi[2], zchunks);
   ++launch_counter();
 }
 
@@ -101,11 +101,11 @@ void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStr
       }
       if constexpr (sizeof(T) == 4) {
         if (p.fp64_policy & kFp64Kinks) {
-          k_stage_pairs<T, KIND, true><<<grid, kPairThreads, 0, st>>>(q);
+          launch_after(k_stage_pairs<T, KIND, true>, grid, kPairThreads, st, q);
           return;
         }
       }
-      k_stage_pairs<T, KIND, false><<<grid, kPairThreads, 0, st>>>(q);
+      launch_after(k_stage_pairs<T, KIND, false>, grid, kPairThreads, st, q);
       return;
     }
   }
@@ -118,15 +118,15 @@ void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStr
       }
       if constexpr (sizeof(T) == 4) {
         if (p.fp64_policy & kFp64Kinks) {
-          k_stage_pairs_up<T, KIND, true><<<grid, kPairThreads, 0, st>>>(q);
+          launch_after(k_stage_pairs_up<T, KIND, true>, grid, kPairThreads, st, q);
           return;
         }
       }
-      k_stage_pairs_up<T, KIND, false><<<grid, kPairThreads, 0, st>>>(q);
+      launch_after(k_stage_pairs_up<T, KIND, false>, grid, kPairThreads, st, q);
       return;
     }
   }
-  k_stage<T, KIND, STAGE_FAST, TX, TY><<<grid, dim3(TX, TY, 1), 0, st>>>(p);
+  launch_after(k_stage<T, KIND, STAGE_FAST, TX, TY>, grid, dim3(TX, TY, 1), st, p);
 }
 
 template <typename T>
