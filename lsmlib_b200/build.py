@@ -37,6 +37,7 @@ SOURCES = {
     "adjoint.cu": ["--fmad=true"],
     "noalloc.cu": ["--fmad=false"],
     "distance.cu": ["--fmad=false"],
+    "host_copy.cu": [],
 }
 
 

@@ -541,18 +541,14 @@ int lsmgpu_batch_grid(lsmgpu_batch* b, int g, long long* offset, int gb[6]) {
 // copy the whole packed phi buffer from/to the host (grid g at its offset)
 int lsmgpu_batch_upload(lsmgpu_batch* b, const void* host) {
   if (!batch_ok(b, "lsmgpu_batch_upload")) return LSMGPU_ERR_NULL_POINTER;
-  return cuda_ok(cudaMemcpy(b->phi, host, (size_t)b->total * b->prec,
-                            cudaMemcpyHostToDevice),
+  return cuda_ok(copy_to_device(b->phi, host, (size_t)b->total * b->prec, b->stream),
                  "lsmgpu_batch_upload")
              ? LSMGPU_SUCCESS
              : LSMGPU_ERR_CUDA;
 }
 int lsmgpu_batch_download(lsmgpu_batch* b, void* host) {
   if (!batch_ok(b, "lsmgpu_batch_download")) return LSMGPU_ERR_NULL_POINTER;
-  if (!cuda_ok(cudaStreamSynchronize(b->stream), "lsmgpu_batch_download"))
-    return LSMGPU_ERR_CUDA;
-  return cuda_ok(cudaMemcpy(host, b->phi, (size_t)b->total * b->prec,
-                            cudaMemcpyDeviceToHost),
+  return cuda_ok(copy_to_host(host, b->phi, (size_t)b->total * b->prec, b->stream),
                  "lsmgpu_batch_download")
              ? LSMGPU_SUCCESS
              : LSMGPU_ERR_CUDA;

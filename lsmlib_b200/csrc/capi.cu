@@ -173,9 +173,7 @@ void* Staging::add(const void* p, const Box& b, int elem, Role role,
     // outputs are copied in too (cells outside the fill box keep their
     // values), unless the routine writes every cell
     if (role != kOutFull &&
-        !cuda_ok(cudaMemcpyAsync(it.dev, it.host, it.bytes,
-                                 cudaMemcpyHostToDevice, st_),
-                 "cudaMemcpyAsync(H2D)")) {
+        !cuda_ok(copy_to_device(it.dev, it.host, it.bytes, st_), "copy to the device")) {
       cudaFreeAsync(it.dev, st_);
       return nullptr;
     }
@@ -189,9 +187,7 @@ bool Staging::finish(const char* routine) {
   bool ok = true;
   for (auto& it : items_) {
     if (it.staged && (it.role & kOut) && ok)
-      ok = cuda_ok(cudaMemcpyAsync(it.host, it.dev, it.bytes,
-                                   cudaMemcpyDeviceToHost, st_),
-                   "cudaMemcpyAsync(D2H)");
+      ok = cuda_ok(copy_to_host(it.host, it.dev, it.bytes, st_), "copy to the host");
   }
   for (auto& it : items_)
     if (it.staged) cudaFreeAsync(it.dev, st_);
@@ -953,6 +949,7 @@ int lsmgpu_free(void* p) {
 int lsmgpu_release_scratch(void) {
   std::lock_guard<std::mutex> lock(g_pool_mu);
   bool ok = cuda_ok(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
+  release_copy_slots();
   for (int d = 0; d < kMaxDevices; d++)
     if (g_pool[d]) ok = cuda_ok(cudaMemPoolTrimTo(g_pool[d], 0), "cudaMemPoolTrimTo") && ok;
   return ok ? LSMGPU_SUCCESS : LSMGPU_ERR_CUDA;

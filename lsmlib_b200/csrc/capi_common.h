@@ -42,6 +42,13 @@ bool covers3(const Box& b, const FillBox& fb, const int w[3], const char* what,
 // lsmgpu_release_scratch() returns them to the driver.
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
 
+// ---- large host copies (host_copy.cu) --------------------------------------------
+// Between host memory and the device, behind the work on st, complete on
+// return.
+cudaError_t copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
+cudaError_t copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st);
+void release_copy_slots();
+
 // ---- staging ----------------------------------------------------------------
 // kOutFull: an output the routine writes completely (no copy in)
 enum Role { kIn = 1, kOut = 2, kInOut = 3, kOutFull = 6 };
