@@ -726,9 +726,9 @@ __device__ __forceinline__ int pair_row_bits(int columns_left) {
   return columns_left <= 8 ? 2 : columns_left <= 16 ? 3 : 4;
 }
 
-template <typename T, bool K64>
+template <typename T, bool K64, bool LMAX = false>
 __device__ __forceinline__ void face_pm_t(const T* u, const FaceConst<T>& k, T& vp, T& vm) {
-  weno5_face<T, sizeof(T) == 4 && K64>(u, k, vp, vm);
+  weno5_face<T, sizeof(T) == 4 && K64, LMAX>(u, k, vp, vm);
 }
 
 template <typename T, int KIND, bool K64>
@@ -901,7 +901,7 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
       } else {
         // the branches (the second cell's y and z faces) keep each block of
         // straight-line code, and so the values live in it, small
-        face_pm_t<T, K64>(u, p.fk[0], xp0, xm1);
+        face_pm_t<T, K64, true>(u, p.fk[0], xp0, xm1);   // shares its maximum with the next
         face_pm_t<T, K64>(u + 1, p.fk[0], xp1, xnext);
         face_pm_t<T, K64>(ya, p.fk[1], yp0, ym0);
         ym1 = T(0);

@@ -80,12 +80,10 @@ __device__ __forceinline__ float vmin(float a, float b) { return fminf(a, b); }
 
 // 2^-(unbiased exponent of x) for a positive normal x
 __device__ __forceinline__ double inv_pow2_of(double x) {
-  const int e = (__double2hiint(x) >> 20) & 0x7ff;
-  return __hiloint2double((2046 - e) << 20, 0);
+  return __hiloint2double(0x7fe00000 - (__double2hiint(x) & 0x7ff00000), 0);
 }
 __device__ __forceinline__ float inv_pow2_of(float x) {
-  const int e = (__float_as_int(x) >> 23) & 0xff;
-  return __int_as_float((254 - e) << 23);
+  return __int_as_float(0x7f000000 - (__float_as_int(x) & 0x7f800000));
 }
 
 // x * inv_pow2_of(x), in [1, 2): the significand with the exponent of 1
@@ -279,12 +277,16 @@ __host__ __device__ inline FaceConst<T> face_const(T inv) {
 // (416 us: four integer instructions for one comparison).
 // When KINK64 is set (FP32 form) a face whose indicators differ by more than
 // a factor 1e3 is recomputed in FP64.
-template <typename T, bool KINK64>
+// LMAX: the eps maximum grouped as max(|V1|, max(|V2|..|V5|)) instead of
+// max(max(|V1|..|V4|), |V5|) -- the same value; a face evaluated with LMAX
+// beside the face one cell on (without) shares the inner four-way maximum.
+template <typename T, bool KINK64, bool LMAX = false>
 __device__ __forceinline__ void weno5_face(const T* u, const FaceConst<T>& k, T& vp, T& vm) {
   const T V1 = u[1] - u[0], V2 = u[2] - u[1], V3 = u[3] - u[2], V4 = u[4] - u[3],
           V5 = u[5] - u[4];
   const T amax =
-      vmax(vmax(vmax(fabs(V1), fabs(V2)), vmax(fabs(V3), fabs(V4))), fabs(V5));
+      LMAX ? vmax(fabs(V1), vmax(vmax(fabs(V2), fabs(V3)), vmax(fabs(V4), fabs(V5))))
+           : vmax(vmax(vmax(fabs(V1), fabs(V2)), vmax(fabs(V3), fabs(V4))), fabs(V5));
   const T m = amax * amax;
   // four times the reference's 1e-6 max(v^2) + tiny, in units of the
   // undivided differences (the floor, reached only where every |D| < 1e-46,
