@@ -88,6 +88,13 @@ __device__ __forceinline__ Time3 ldcg(const Time3* t) {
   return Time3{__ldcg(&t->a), __ldcg(&t->b), __ldcg(&t->c)};
 }
 
+// What an evaluation reads of a point: its value and the first level of its
+// time, with kKeyFront for a front point and kKeyOutside outside the domain
+// (times are >= 0) -- one 16-byte load in place of the value, the time and
+// the status byte.
+constexpr double kKeyFront = -1.0, kKeyOutside = -2.0;
+__device__ __forceinline__ bool key_inside(double k) { return k > -1.5; }
+
 // linear index of the k-th point (k = 1, 2) from o in slot q's direction
 __device__ __forceinline__ long nb_index(long o, const long s[3], int q, int k) {
   return o + ((q & 1) ? k : -k) * s[q >> 1];
@@ -339,7 +346,8 @@ __device__ __forceinline__ double fmm_root(double A, double B, double disc) {
 
 // The threshold advances by this many of the smallest spacing per step.  A
 // longer step takes fewer passes and revises its points more often: 6 cells
-// where the lists leave threads idle and a pass costs its latency (301x237,
+// where the lists leave threads idle and a pass costs its latency (measured
+// before a point's value and key became one load: 301x237,
 // order 1: 571 passes of 10.5 us with 2 cells, 405 of 11.3 with 6; 64^3: 256
 // and 228 of 14.0), 2 where they fill the GPU (128x112x120, order 2: 16.8 ms
 // against 20.6 with 6).
@@ -360,8 +368,7 @@ constexpr double kDeltaCells = 2.0, kDeltaCellsSmall = 6.0;
 // solver the point's input.  Neighbours off the grid
 // are left out, as the reference's bounds checks do.
 template <int ORDER, bool EIK>
-__device__ __noinline__ bool fmm_point(const double* d, const Time3* tm, const unsigned char* st,
-                                       long o, int c0, int c1, int c2, int nx, int ny, int nz,
+__device__ __noinline__ bool fmm_point(const double2* vk, const Time3* tm, long o, int c0, int c1, int c2, int nx, int ny, int nz,
                                        double i2x, double i2y, double i2z, Eik E, Update* U) {
   const int c[3] = {c0, c1, c2}, n[3] = {nx, ny, nz};
   const long s[3] = {1L, (long)nx, (long)nx * ny};
@@ -369,7 +376,7 @@ __device__ __noinline__ bool fmm_point(const double* d, const Time3* tm, const u
   Stencil nb;
   // every load first, at in-range addresses (the point itself stands in
   // for a neighbour off the grid), so that they are in flight together
-  unsigned char s1[6], s2[6];
+  double s1[6], s2[6];
   bool in1[6], in2[6];
 #pragma unroll
   for (int q = 0; q < 6; q++) {
@@ -377,39 +384,41 @@ __device__ __noinline__ bool fmm_point(const double* d, const Time3* tm, const u
     const int sg = (q & 1) ? 1 : -1;
     in1[q] = c[dir] + sg >= 0 && c[dir] + sg < n[dir];
     const long o1 = in1[q] ? o + sg * s[dir] : o;
-    s1[q] = st[o1];
-    nb.v1[q] = __ldcg(d + o1);
+    const double2 p1 = __ldcg(vk + o1);
+    s1[q] = p1.y;
+    nb.v1[q] = p1.x;
     nb.t1[q] = ldcg(tm + o1);
     if (ORDER == 2) {
       in2[q] = in1[q] && c[dir] + 2 * sg >= 0 && c[dir] + 2 * sg < n[dir];
       const long o2 = in2[q] ? o + 2 * sg * s[dir] : o;
-      s2[q] = st[o2];
-      nb.v2[q] = __ldcg(d + o2);
+      const double2 p2 = __ldcg(vk + o2);
+      s2[q] = p2.y;
+      nb.v2[q] = p2.x;
       nb.t2[q] = ldcg(tm + o2);
     }
   }
   nb.has1 = nb.front1 = nb.has2 = nb.front2 = 0;
 #pragma unroll
   for (int q = 0; q < 6; q++) {
-    const bool k1 = in1[q] && s1[q] != kOutside && fabs(nb.v1[q]) <= DBL_MAX;
+    const bool k1 = in1[q] && key_inside(s1[q]) && fabs(nb.v1[q]) <= DBL_MAX;
     if (!k1) {
       nb.v1[q] = DBL_MAX;
       nb.t1[q] = Time3{INFINITY, INFINITY, INFINITY};
       continue;
     }
     nb.has1 |= 1 << q;
-    if (s1[q] == kFront) {
+    if (s1[q] < 0) {
       nb.front1 |= 1 << q;
       nb.t1[q] = Time3{INFINITY, INFINITY, INFINITY};
     }
     if (ORDER == 2) {
-      const bool k2 = in2[q] && s2[q] != kOutside && fabs(nb.v2[q]) <= DBL_MAX;
+      const bool k2 = in2[q] && key_inside(s2[q]) && fabs(nb.v2[q]) <= DBL_MAX;
       if (!k2) {
         nb.v2[q] = DBL_MAX;
         continue;
       }
       nb.has2 |= 1 << q;
-      if (s2[q] == kFront) nb.front2 |= 1 << q;
+      if (s2[q] < 0) nb.front2 |= 1 << q;
     }
   }
   if (!nb.has1) return false;
@@ -507,7 +516,8 @@ __device__ __noinline__ bool fmm_point(const double* d, const Time3* tm, const u
 // negative discriminant and 0.03 % a lowered time, but each took 2.6 roots (a
 // square root and a division) to decide which neighbours come before the
 // value, and some 3000 instructions in a row.  Here
-//   - only the first level of a time is read; the others when two tie;
+//   - of a neighbour only its value and the first level of its time are read,
+//     as one pair; the other levels when two tie;
 //   - "a neighbour of key x comes before |value|" is read off the sign of the
 //     quadratic at x where it is clear of rounding, and the root is taken once
 //     at the end;
@@ -515,15 +525,16 @@ __device__ __noinline__ bool fmm_point(const double* d, const Time3* tm, const u
 //     negative or undefined discriminant, a vanishing linear term, for the
 //     Eikonal solver a negative value) is left to fmm_point.
 // Returns 1 with the update, 0 for a point no neighbour reaches, -1 for a
-// point left to fmm_point.  The arithmetic of the coefficients and of the
-// root is fmm_coeffs' and fmm_root's.
+// point left to fmm_point; ``readers``: the free points whose stencil reads
+// this one (bit ORDER * slot, and at second order the next for the point
+// behind).  The arithmetic of the coefficients and of the root is fmm_coeffs'
+// and fmm_root's.
 template <int ORDER, bool EIK>
-__device__ __forceinline__ int fmm_point_fast(const double* d, const Time3* tm,
-                                              const unsigned char* st, long o, const int c[3],
-                                              const int n[3], const long s[3],
-                                              const double i2[3], const Eik& E, Update& U) {
+__device__ __forceinline__ int fmm_point_fast(const double2* vk, const Time3* tm, long o,
+                                              const int c[3], const int n[3], const long s[3],
+                                              const double i2[3], const Eik& E, Update& U,
+                                              unsigned& readers) {
   double v1[6], k1[6], v2[6], k2[6];
-  unsigned char s1[6], s2[6];
   unsigned in1 = 0, in2 = 0;
   const double cterm = EIK ? 1 / E.speed[o] / E.speed[o] : 1.0;
   // every load first, at in-range addresses, as in fmm_point
@@ -534,16 +545,16 @@ __device__ __forceinline__ int fmm_point_fast(const double* d, const Time3* tm,
     const bool i1 = a1 >= 0 && a1 < n[dir];
     const long o1 = i1 ? o + sg * s[dir] : o;
     in1 |= (unsigned)i1 << q;
-    s1[q] = st[o1];
-    v1[q] = __ldcg(d + o1);
-    k1[q] = __ldcg(&tm[o1].a);
+    const double2 p1 = __ldcg(vk + o1);
+    v1[q] = p1.x;
+    k1[q] = p1.y;
     if (ORDER == 2) {
       const bool b2 = a2 >= 0 && a2 < n[dir];
       const long o2 = b2 ? o + 2 * sg * s[dir] : o;
       in2 |= (unsigned)b2 << q;
-      s2[q] = st[o2];
-      v2[q] = __ldcg(d + o2);
-      k2[q] = __ldcg(&tm[o2].a);
+      const double2 p2 = __ldcg(vk + o2);
+      v2[q] = p2.x;
+      k2[q] = p2.y;
     }
   }
   // masks, a bit per slot: in the update so far (the fronts), waiting (the
@@ -551,17 +562,20 @@ __device__ __forceinline__ int fmm_point_fast(const double* d, const Time3* tm,
   // (a front) or once accepted before the trigger; a bit per axis: the plus
   // side is the smaller
   unsigned incl = 0, rem = 0, sec = 0, dyn = 0, plus_less = 0;
+  readers = 0;
 #pragma unroll
   for (int q = 0; q < 6; q++) {
-    const bool has = (in1 >> q & 1) && s1[q] != kOutside && fabs(v1[q]) <= DBL_MAX;
-    const bool front = has && s1[q] == kFront;
+    const bool has = (in1 >> q & 1) && key_inside(k1[q]) && fabs(v1[q]) <= DBL_MAX;
+    const bool front = has && k1[q] < 0;
+    readers |= (unsigned)((in1 >> q & 1) && !(k1[q] < 0)) << (q * ORDER);
     incl |= (unsigned)front << q;
     rem |= (unsigned)(has && !front) << q;
     if (!(has && !front)) k1[q] = INFINITY;
     if (ORDER == 2) {
-      const bool has2 = has && (in2 >> q & 1) && s2[q] != kOutside &&
+      const bool has2 = has && (in2 >> q & 1) && key_inside(k2[q]) &&
                         fabs(v2[q]) <= fabs(v1[q]);
-      const bool front2 = has2 && s2[q] == kFront;
+      const bool front2 = has2 && k2[q] < 0;
+      readers |= (unsigned)((in2 >> q & 1) && !(k2[q] < 0)) << (2 * q + 1);
       sec |= (unsigned)front2 << q;
       dyn |= (unsigned)(has2 && !front2) << q;
     }
@@ -749,6 +763,7 @@ struct Lists {
   int* stamp;                // pass that last queued a point
   int* pending;              // two lists of n points (by epoch parity)
   int* pend_stamp;           // epoch + 1 that last queued a point
+  double2* vk;               // per point: value and key (kKeyFront, kKeyOutside)
   double* new_d;             // per slot of the active list beyond each thread's
   Time3* new_t;              //   first: the evaluated value, time and whether
   unsigned char* new_f;      //   to store them
@@ -773,14 +788,18 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
   return v;
 }
 
-// The first active list: the free points next to the front.
-__global__ void k_fmm_seed(const unsigned char* st, int nx, int ny, int nz, Lists L,
+// The points' pairs, and the first active list: the free points next to the
+// front.
+__global__ void k_fmm_seed(const double* d, const unsigned char* st, int nx, int ny, int nz, Lists L,
                            Ctrl* ctrl) {
   const long n = (long)nx * ny * nz;
   const long s[3] = {1L, (long)nx, (long)nx * ny};
   const int nn[3] = {nx, ny, nz};
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < n;
        o += (long)gridDim.x * blockDim.x) {
+    L.vk[o] = make_double2(d[o], st[o] == kFront     ? kKeyFront
+                                 : st[o] == kOutside ? kKeyOutside
+                                                     : INFINITY);
     if (st[o] != kFree) continue;
     int c[3];
     point_coords(o, nx, ny, c);
@@ -808,8 +827,12 @@ __global__ void k_fmm_seed(const unsigned char* st, int nx, int ny, int nz, List
 constexpr int kTailFraction = 4;
 
 // Threads of a block of k_fmm_march, one block per SM (or of the one
-// cluster): 122 registers at order 1, 168 at order 2.
-__host__ __device__ constexpr int march_threads(int order) { return order == 1 ? 512 : 384; }
+// cluster): 128 registers a thread, 168 at order 2 over the GPU (with 512
+// threads there 17.4 ms for 16.7 at 128x112x120; in the cluster 6.2 for 6.5 at
+// 301x237).
+__host__ __device__ constexpr int march_threads(int order, bool cluster) {
+  return order == 1 || cluster ? 512 : 384;
+}
 constexpr int kClusterBlocks = 8;
 
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;   // +infinity
@@ -929,16 +952,18 @@ __device__ __forceinline__ int2 reserve(int mine, int mine2, int* count, int* co
 // 24.9 ms a call from host arrays; 301x237, two extension fields: 11.9 ms).
 // Here the readers are queued by the thread that found the change, beside
 // the evaluation, a thread keeps its first slot's result in registers, the
-// stamps of a point's readers are exchanged together, and the warps of a
-// short list are spread over the SMs: 10 to 15 us a pass where the lists are
-// short (half of it the evaluation, the rest the two barriers and the queue),
-// 35 at 68,000 points a pass.
+// stamps of a point's readers are exchanged together, the warps of a short
+// list are spread over the SMs, and a neighbour is one 16-byte load (value,
+// time and status apart were a third more loads each, scattered over as many
+// sectors: 35 us a pass at 68,000 points, 10.5 at 1,700).  9 to 14 us a pass
+// where the lists are short (half of it the evaluation, the rest the two
+// barriers and the queue), 31 at 68,000 points.
 // Lists that fit one cluster's threads run on 8 SMs, whose barrier is a
 // hardware one.
 template <int ORDER, bool EIK, bool CLUSTER>
-__global__ void __launch_bounds__(march_threads(ORDER), 1)
-k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int nz, double i2x,
-            double i2y, double i2z, Lists L, Ctrl* ctrl, ExtSet X, Eik E, double delta,
+__global__ void __launch_bounds__(march_threads(ORDER, CLUSTER), 1)
+k_fmm_march(Time3* tm, int nx, int ny, int nz, double i2x, double i2y, double i2z, Lists L,
+            Ctrl* ctrl, ExtSet X, Eik E, double delta,
             int max_passes) {
   constexpr int kReaders = 6 * ORDER;
   __shared__ Room room;
@@ -949,6 +974,7 @@ k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int n
   } c_;
   __shared__ int s_ok;
   const long n = (long)nx * ny * nz;
+  double2* const vk = L.vk;
   const int lane = threadIdx.x & 31;
   const int nb = (int)gridDim.x, bid = (int)blockIdx.x;
   const int total = nb * (int)blockDim.x;
@@ -997,16 +1023,17 @@ k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int n
         o = __ldcg(cur + w);
         // only free points are ever queued; the value and time of the
         // point itself are loaded beside its stencil
-        const double old = __ldcg(d + o);
-        const Time3 told = ldcg(tm + o);
+        const double2 self = __ldcg(vk + o);
+        const double old = self.x, told_b = __ldcg(&tm[o].b);
         int c[3];
         point_coords(o, nx, ny, c);
         Update U;
-        int reached = fmm_point_fast<ORDER, EIK>(d, tm, st, o, c, nn, s, i2, E, U);
+        unsigned cand;
+        int reached = fmm_point_fast<ORDER, EIK>(vk, tm, o, c, nn, s, i2, E, U, cand);
         if (reached < 0) {
           Update slow;
-          reached = fmm_point<ORDER, EIK>(d, tm, st, o, c[0], c[1], c[2], nx, ny, nz, i2x, i2y,
-                                          i2z, E, &slow);
+          reached = fmm_point<ORDER, EIK>(vk, tm, o, c[0], c[1], c[2], nx, ny, nz, i2x, i2y, i2z,
+                                          E, &slow);
           U = slow;
         }
         double val = U.val;
@@ -1025,7 +1052,9 @@ k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int n
         } else if (!EIK && X.nf) {
           ext_changed = fmm_ext(U, i2, X, o, s);
         }
-        const bool store = ext_changed || !(val == old && tequal(tv, told));
+        // (the third level counts where the second does)
+        const bool store = ext_changed || !(val == old && tv.a == self.y && tv.b == told_b &&
+                                            (tv.b == -1.0 || tv.c == __ldcg(&tm[o].c)));
         if (base == 0) {
           f_first = store;
           o_first = (int)o;
@@ -1039,17 +1068,6 @@ k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int n
         // the free points whose stencil reads this one, where the change is
         // visible: the value is finite before or after, or a field changed
         if (store && (ext_changed || fabs(old) <= DBL_MAX || fabs(val) <= DBL_MAX)) {
-          unsigned cand = 0;
-#pragma unroll
-          for (int q = 0; q < 6; q++) {
-            const int dir = q >> 1, sg = (q & 1) ? 1 : -1;
-#pragma unroll
-            for (int r = 1; r <= ORDER; r++) {
-              const int cr = c[dir] + r * sg;
-              if (cr >= 0 && cr < nn[dir] && st[o + r * sg * s[dir]] == kFree)
-                cand |= 1u << (q * ORDER + r - 1);
-            }
-          }
           // the exchanges go out together: predicated, without branches
           int was[kReaders];
 #pragma unroll
@@ -1079,8 +1097,9 @@ k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int n
       int o = 0;
       if (w < filter) {
         o = __ldcg(src + w);
-        const double t = __ldcg(&tm[o].a);
-        if (!(fabs(__ldcg(d + o)) <= DBL_MAX)) {   // not reached since
+        const double2 self = __ldcg(vk + o);
+        const double t = self.y;
+        if (!(fabs(self.x) <= DBL_MAX)) {   // not reached since
           if (t <= T) {
             go = atomicExch(L.stamp + o, pass + 2) != pass + 2;
           } else if (t < INFINITY) {
@@ -1108,14 +1127,15 @@ k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int n
     }
     if (!march_barrier<CLUSTER>(ctrl, gen, &s_ok)) return;
     if (f_first) {
-      d[o_first] = d_first;
+      vk[o_first] = make_double2(d_first, t_first.a);
       tm[o_first] = t_first;
     }
     for (int w = slot + total; w < count; w += total)
       if (L.new_f[w]) {
         const int o = __ldcg(cur + w);
-        d[o] = L.new_d[w];
-        tm[o] = L.new_t[w];
+        const Time3 t = L.new_t[w];
+        vk[o] = make_double2(L.new_d[w], t.a);
+        tm[o] = t;
       }
     if (!march_barrier<CLUSTER>(ctrl, gen, &s_ok)) return;
     // thread 0 of each block: the threshold control, from the same words in
@@ -1158,13 +1178,19 @@ k_fmm_march(double* d, Time3* tm, const unsigned char* st, int nx, int ny, int n
   }
 }
 
-// free points no front reached: the reference's default value -1 (distance
+// The values of the free points; those no front reached take the reference's
+// default value -1 (distance
 // and extension fields), or the Eikonal solver's input
-__global__ void k_fmm_unreached(double* d, const unsigned char* st, long n, ExtSet X,
-                                const double* phi0) {
+__global__ void k_fmm_finish(double* d, const double2* vk, const unsigned char* st, long n,
+                             ExtSet X, const double* phi0) {
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < n;
        o += (long)gridDim.x * blockDim.x)
-    if (st[o] == kFree && !(fabs(d[o]) <= DBL_MAX)) {
+    if (st[o] == kFree) {
+      const double v = vk[o].x;
+      if (fabs(v) <= DBL_MAX) {
+        d[o] = v;
+        continue;
+      }
       d[o] = phi0 ? phi0[o] : -1.0;
       for (int f = 0; f < X.nf; f++) X.ext[f][o] = -1.0;
     }
@@ -1188,7 +1214,7 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
   // points of a typical list: two per point of the grid's largest cross-section
   const int longest = nx > ny ? (nx > nz ? nx : nz) : (ny > nz ? ny : nz);
   const long band = 2 * n / longest;
-  Lists L{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  Lists L{};
   Ctrl* ctrl = nullptr;
   const size_t un = (size_t)n;
   bool ok = cuda_ok(pool_alloc((void**)&status, un, st), R) &&
@@ -1197,6 +1223,7 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
             cuda_ok(pool_alloc((void**)&L.pending, 2 * un * sizeof(int), st), R) &&
             cuda_ok(pool_alloc((void**)&L.stamp, un * sizeof(int), st), R) &&
             cuda_ok(pool_alloc((void**)&L.pend_stamp, un * sizeof(int), st), R) &&
+            cuda_ok(pool_alloc((void**)&L.vk, un * sizeof(double2), st), R) &&
             cuda_ok(pool_alloc((void**)&L.new_d, un * sizeof(double), st), R) &&
             cuda_ok(pool_alloc((void**)&L.new_t, un * sizeof(Time3), st), R) &&
             cuda_ok(pool_alloc((void**)&L.new_f, un, st), R) &&
@@ -1223,7 +1250,7 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     else
       k_fmm_front<<<grid3, blk, 0, st>>>(dd, tm, status, dp, dm, nx, ny, nz, dx[0], dx[1],
                                          dx[2], X);
-    k_fmm_seed<<<elem_blocks, 256, 0, st>>>(status, nx, ny, nz, L, ctrl);
+    k_fmm_seed<<<elem_blocks, 256, 0, st>>>(dd, status, nx, ny, nz, L, ctrl);
     launch_counter() += 2;
     ok = cuda_ok(cudaGetLastError(), R);
   }
@@ -1235,8 +1262,8 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
   }
   // One cluster while the lists fit its threads, else one block per SM of a
   // cooperative launch; and the threshold's step
-  const bool cluster = band <= kClusterBlocks * march_threads(2);
-  const bool small = cluster || 4 * band <= (long)sms * march_threads(order);
+  const bool cluster = band <= kClusterBlocks * 384;
+  const bool small = cluster || 4 * band <= (long)sms * march_threads(order, false);
   const double delta = (small ? kDeltaCellsSmall : kDeltaCells) * hmin;
   // (passes in whole batches of 32)
   int passes = (int)((max_passes + 31) / 32 * 32);
@@ -1254,8 +1281,8 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     Eik es = E;
     double step = delta;
     int mx = nx, my = ny, mz = nz;
-    void* args[] = {&dd, &tm, &status, &mx, &my,   &mz,   &i2[0], &i2[1],
-                    &i2[2], &L, &ctrl,   &xs, &es, &step, &passes};
+    void* args[] = {&tm, &mx, &my, &mz, &i2[0], &i2[1], &i2[2], &L, &ctrl, &xs, &es, &step,
+                    &passes};
     cudaLaunchAttribute at{};
     at.id = cluster ? cudaLaunchAttributeClusterDimension : cudaLaunchAttributeCooperative;
     if (cluster) {
@@ -1266,7 +1293,7 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(cluster ? kClusterBlocks : sms);
-    cfg.blockDim = dim3(march_threads(order));
+    cfg.blockDim = dim3(march_threads(order, cluster));
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
@@ -1284,12 +1311,12 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     }
   }
   if (ok) {
-    k_fmm_unreached<<<elem_blocks, 256, 0, st>>>(dd, status, n, X, E.phi0);
+    k_fmm_finish<<<elem_blocks, 256, 0, st>>>(dd, L.vk, status, n, X, E.phi0);
     ++launch_counter();
     ok = cuda_ok(cudaGetLastError(), R);
   }
   for (void* q : {(void*)status, (void*)tm, (void*)L.active, (void*)L.pending,
-                  (void*)L.stamp, (void*)L.pend_stamp, (void*)L.new_d, (void*)L.new_t,
+                  (void*)L.stamp, (void*)L.pend_stamp, (void*)L.vk, (void*)L.new_d, (void*)L.new_t,
                   (void*)L.new_f, (void*)ctrl})
     if (q) cudaFreeAsync(q, st);
   if (passes_out) *passes_out = h_ctrl.pass;
