@@ -542,14 +542,16 @@ int lsmgpu_batch_grid(lsmgpu_batch* b, int g, long long* offset, int gb[6]) {
 int lsmgpu_batch_upload(lsmgpu_batch* b, const void* host) {
   if (!batch_ok(b, "lsmgpu_batch_upload")) return LSMGPU_ERR_NULL_POINTER;
   return cuda_ok(copy_to_device(b->phi, host, (size_t)b->total * b->prec, b->stream),
-                 "lsmgpu_batch_upload")
+                 "lsmgpu_batch_upload") &&
+                 cuda_ok(cudaStreamSynchronize(b->stream), "lsmgpu_batch_upload")
              ? LSMGPU_SUCCESS
              : LSMGPU_ERR_CUDA;
 }
 int lsmgpu_batch_download(lsmgpu_batch* b, void* host) {
   if (!batch_ok(b, "lsmgpu_batch_download")) return LSMGPU_ERR_NULL_POINTER;
   return cuda_ok(copy_to_host(host, b->phi, (size_t)b->total * b->prec, b->stream),
-                 "lsmgpu_batch_download")
+                 "lsmgpu_batch_download") &&
+                 cuda_ok(cudaStreamSynchronize(b->stream), "lsmgpu_batch_download")
              ? LSMGPU_SUCCESS
              : LSMGPU_ERR_CUDA;
 }

@@ -43,8 +43,8 @@ bool covers3(const Box& b, const FillBox& fb, const int w[3], const char* what,
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
 
 // ---- large host copies (host_copy.cu) --------------------------------------------
-// Between host memory and the device, behind the work on st, complete on
-// return.
+// Between host memory and the device, behind the work on st.  A large one is
+// complete on return; another is a cudaMemcpyAsync on st.
 cudaError_t copy_to_host(void* host, const void* dev, size_t bytes, cudaStream_t st);
 cudaError_t copy_to_device(void* dev, const void* host, size_t bytes, cudaStream_t st);
 void release_copy_slots();

@@ -78,7 +78,7 @@ bool pageable(const void* host) {
   return at.type == cudaMemoryTypeUnregistered;
 }
 
-// behind the work on st; complete on return
+// behind the work on st: in pieces, complete on return, or plainly on st
 cudaError_t copy(char* host, char* dev, size_t bytes, bool to_host, cudaStream_t st) {
   int device = 0;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -87,10 +87,8 @@ cudaError_t copy(char* host, char* dev, size_t bytes, bool to_host, cudaStream_t
       cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
       !pageable(host) || !lock.try_lock() || !have_slots(device)) {
     cudaGetLastError();
-    const cudaError_t e =
-        to_host ? cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st)
-                : cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
-    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    return to_host ? cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st)
+                   : cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
   }
   cudaError_t e = cudaEventRecord(g_slots.ready, st);
   if (e != cudaSuccess) return e;
