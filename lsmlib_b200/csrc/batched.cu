@@ -86,11 +86,13 @@ template <typename T, int TX, int TY, int STAGING>
 __device__ __forceinline__ void batch_tile(const StageParams<T>& p, int bx, int by, int bz,
                                            int policy) {
   if constexpr (STAGING == kPairStaging) {
-    __shared__ __align__(16) T tile[2][TY + 6][TX + 8];
+    // (a narrow last column takes taller tiles, so its last items are empty)
+    __shared__ __align__(16) T tile[2][TX * TY / 8 + 6][TX + 8];
     if (sizeof(T) == 4 && (policy & kFp64Kinks))
-      stage_tile_pairs_up<T, kStageAdvectConst, sizeof(T) == 4, TX, TY>(p, bx, by, bz, tile);
+      stage_tile_pairs_up<T, kStageAdvectConst, sizeof(T) == 4, TX, TY, false, true>(p, bx, by,
+                                                                                    bz, tile);
     else
-      stage_tile_pairs_up<T, kStageAdvectConst, false, TX, TY>(p, bx, by, bz, tile);
+      stage_tile_pairs_up<T, kStageAdvectConst, false, TX, TY, false, true>(p, bx, by, bz, tile);
   } else {
     __shared__ T tile[2][TY + 6][TX + 6];
     stage_tile<T, kStageAdvectConst, true, TX, TY, STAGING>(p, bx, by, bz, tile);

@@ -722,8 +722,9 @@ constexpr int kPairPX = 4;
 // one column in 33 (9 at 256) would otherwise run with 1 of its 32 columns.
 constexpr int kPairTX = 32, kPairTY = 8, kPairThreads = 128;
 constexpr int kPairRows = kPairThreads / 4 + 6;   // rows of the tallest tile and its halo
+template <int TX = kPairTX>
 __device__ __forceinline__ int pair_row_bits(int columns_left) {
-  return columns_left <= 8 ? 2 : columns_left <= 16 ? 3 : 4;
+  return columns_left <= 8 ? 2 : TX == 16 || columns_left <= 16 ? 3 : 4;
 }
 
 template <typename T, bool K64, bool LMAX = false>
@@ -738,7 +739,7 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
   using T2 = typename Pair2<T>::type;
   constexpr int PX = kPairPX;
   const int x0 = p.fb.lo[0] + bx * kPairTX;
-  const int lp = pair_row_bits(p.fb.hi[0] - x0 + 1);
+  const int lp = pair_row_bits<kPairTX>(p.fb.hi[0] - x0 + 1);
   const int NP = 1 << lp, TX = 2 * NP, TY = kPairThreads >> lp;
   const int tid = threadIdx.x, t = tid & (NP - 1), ty = tid >> lp;
   const int j0 = p.fb.lo[1] + by * TY;
@@ -960,24 +961,25 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
 // FP32 without the FP64 kink recomputation, where the two cells' sides of
 // an axis are one packed FP32x2 evaluation (weno5_side2).
 // BAND: the FP64 band form (out_alt written as well).  NARROW: the last
-// column of tiles may take shorter rows (pair_row_bits), block of
-// kPairThreads threads.
+// column of tiles may take shorter rows (pair_row_bits) of as many more
+// rows.
 template <typename T, int KIND, bool K64, int TX_, int TY_, bool BAND = false, bool NARROW = false>
 __device__ __forceinline__ void stage_tile_pairs_up(
     const StageParams<T>& p, int bx, int by, int bz,
-    T (*tile)[NARROW ? kPairRows : TY_ + 6][TX_ + 8]) {
+    T (*tile)[NARROW ? TX_ * TY_ / 8 + 6 : TY_ + 6][TX_ + 8]) {
   using T2 = typename Pair2<T>::type;
   // (no lane exchange: a row of TX/2 >= 4 threads of any width works)
   static_assert(TX_ % 2 == 0 && TX_ / 2 >= 4, "strip roles need four threads per row");
   static_assert(TY_ >= 3, "the y strips need three rows at each end");
-  static_assert(!NARROW || (TX_ == kPairTX && TY_ == kPairTY), "narrow columns: 32 x 8 tiles");
+  static_assert(!NARROW || TX_ == 32 || TX_ == 16, "narrow columns: 32 or 16 wide tiles");
   constexpr int PX = kPairPX;
   const int x0 = p.fb.lo[0] + bx * TX_;
-  const int lp = NARROW ? pair_row_bits(p.fb.hi[0] - x0 + 1) : 0;
+  const int lp = NARROW ? pair_row_bits<TX_>(p.fb.hi[0] - x0 + 1) : 0;
   const int NP = NARROW ? 1 << lp : TX_ / 2;
-  const int TX = 2 * NP, TY = NARROW ? kPairThreads >> lp : TY_;
-  const int t = NARROW ? threadIdx.x & (NP - 1) : threadIdx.x;
-  const int ty = NARROW ? threadIdx.x >> lp : threadIdx.y;
+  const int TX = 2 * NP, TY = NARROW ? (TX_ / 2 * TY_) >> lp : TY_;
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  const int t = NARROW ? tid & (NP - 1) : threadIdx.x;
+  const int ty = NARROW ? tid >> lp : threadIdx.y;
   const int j0 = p.fb.lo[1] + by * TY;
   if (NARROW && j0 > p.fb.hi[1]) return;   // a narrow column has fewer tiles
   const int c0 = 2 * t;
