@@ -310,7 +310,10 @@ __device__ __forceinline__ void weno5_face(const T* u, const FaceConst<T>& k, T&
       }
     }
   }
-  const T sc = inv_pow2_of(eps), es = mantissa_of(eps);   // es = eps * sc
+  // (the product and mantissa_of(eps) are the same number; by integer
+  // operations here the stages at 256^3 took 368.7 and 382.3 us
+  // (reinitialization, normal speed), by the product 366.1 and 379.9)
+  const T sc = inv_pow2_of(eps), es = eps * sc;
   const T qa = fmaT(Sa, sc, es), qb = fmaT(Sb, sc, es), qc = fmaT(Sc, sc, es);
   const T Qa = qa * qa, Qb = qb * qb, Qc = qc * qc;
   const T Pbc = Qb * Qc, Pac = Qa * Qc, Pab = Qa * Qb;
