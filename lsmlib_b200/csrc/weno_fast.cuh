@@ -271,7 +271,7 @@ __host__ __device__ inline FaceConst<T> face_const(T inv) {
 // 62 FP64 instructions a face (57 for the second of two faces one cell apart)
 // against 67 (61) with the indicators formed from V directly.  FP64 stages
 // at 256^3 (fill box), with the right-hand sides of upwind_max0 (stage.cuh):
-// reinitialization 403 -> 373 us, normal speed 414 -> 388 us.  Two faces
+// reinitialization 403 -> 366 us, normal speed 414 -> 380 us.  Two faces
 // written in step, operation by operation, was slower (386 us: both faces'
 // values are live at once), as were eps maxima compared as 64-bit integers
 // (416 us: four integer instructions for one comparison).
@@ -381,11 +381,17 @@ __device__ __forceinline__ void weno5_face2(const float2* u, float inv, float2& 
   const float2 A = mul2(Pbc, sub2(ta, tb)), B = mul2(Pab, sub2(tb, tc));
   const float2 num_m = fma2(f2(1.5f), B, A);
   const float2 num_p = fma2(f2(-1.5f), A, mul2(f2(-1.0f), B));   // negated
-  // three times the middle candidates
-  const float2 p2m = fma2(f2(3.0f), V3, fma2(f2(0.5f), e2, e3));
-  const float2 p2p = fma2(f2(-1.5f), rb, p2m);
-  const float2 sm = fma2(f2(3.0f), Pab, fma2(f2(6.0f), Pac, Pbc));
-  const float2 sp = fma2(f2(3.0f), Pbc, fma2(f2(6.0f), Pac, Pab));
+  // the middle candidates with V3 as it is and the weight sums three times
+  // over: a factor 1/3 on the result instead has a rounding error of its own,
+  // the same one in every derivative of an axis (mean error against FP64 of 20
+  // steps of reinitialization at 160x144x130, stochastic rounding: 3.25e-8 by
+  // that factor, 3.22e-8 so; the stages at 256^3 237.5 and 238, normal speed
+  // 237.7 and 239.9 us)
+  const float2 p2m = fma2(f2(1.0f / 3.0f), fma2(f2(0.5f), e2, e3), V3);
+  const float2 p2p = fma2(f2(-0.5f), rb, p2m);
+  const float2 p18 = mul2(f2(18.0f), Pac);
+  const float2 sm = fma2(f2(3.0f), Pbc, fma2(f2(9.0f), Pab, p18));
+  const float2 sp = fma2(f2(3.0f), Pab, fma2(f2(9.0f), Pbc, p18));
   // reciprocals: per-lane seeds, one packed Newton-Raphson step (rcp_nr)
   float2 rm, rp;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rm.x) : "f"(sm.x));
@@ -394,9 +400,8 @@ __device__ __forceinline__ void weno5_face2(const float2* u, float inv, float2& 
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rp.y) : "f"(sp.y));
   rm = fma2(rm, fma2(mul2(f2(-1.0f), sm), rm, f2(1.0f)), rm);
   rp = fma2(rp, fma2(mul2(f2(-1.0f), sp), rp, f2(1.0f)), rp);
-  const float2 i3 = f2(inv * (1.0f / 3.0f));
-  vm = mul2(fma2(num_m, rm, p2m), i3);
-  vp = mul2(fma2(num_p, rp, p2p), i3);
+  vm = mul2(fma2(num_m, rm, p2m), f2(inv));
+  vp = mul2(fma2(num_p, rp, p2p), f2(inv));
 }
 
 // weno5_side_fast<float> for two independent sides at once, one per lane of
@@ -423,6 +428,8 @@ __device__ __forceinline__ float2 weno5_side2(const float2* D, float inv) {
   const float2 Q1 = mul2(q1, q1), Q2 = mul2(q2, q2), Q3 = mul2(q3, q3);
   const float2 P23 = mul2(Q2, Q3), P13 = mul2(Q1, Q3), P12 = mul2(Q1, Q2);
   const float2 num = fma2(f2(1.5f), mul2(P12, sub2(tb, tc)), mul2(P23, sub2(ta, tb)));
+  // (scaled as in weno5_face2 the velocity arrays take 240 us at 256^3 for 227,
+  // and the error against FP64 is the same to 0.2 %)
   const float2 den = fma2(f2(3.0f), P12, fma2(f2(6.0f), P13, P23));
   const float2 p2 = fma2(f2(3.0f), D3, fma2(f2(0.5f), e2, e3));
   float2 r;
