@@ -383,10 +383,10 @@ __device__ __forceinline__ void weno5_face2(const float2* u, float inv, float2& 
   const float2 num_p = fma2(f2(-1.5f), A, mul2(f2(-1.0f), B));   // negated
   // the middle candidates with V3 as it is and the weight sums three times
   // over: a factor 1/3 on the result instead has a rounding error of its own,
-  // the same one in every derivative of an axis (mean error against FP64 of 20
-  // steps of reinitialization at 160x144x130, stochastic rounding: 3.25e-8 by
-  // that factor, 3.22e-8 so; the stages at 256^3 237.5 and 238, normal speed
-  // 237.7 and 239.9 us)
+  // the same one in every derivative of an axis (mean error against FP64 at
+  // |phi| < 5 dx, 80 steps with their reinitialization at 160x144x130: 1.3e-8
+  // by that factor, 7.8e-9 so; the stages at 256^3 237.5 and 238, normal speed
+  // 237.7 and 240 us).  V3 apart as in weno5_side2 takes 240.3 for 238.
   const float2 p2m = fma2(f2(1.0f / 3.0f), fma2(f2(0.5f), e2, e3), V3);
   const float2 p2p = fma2(f2(-0.5f), rb, p2m);
   const float2 p18 = mul2(f2(18.0f), Pac);
@@ -428,15 +428,17 @@ __device__ __forceinline__ float2 weno5_side2(const float2* D, float inv) {
   const float2 Q1 = mul2(q1, q1), Q2 = mul2(q2, q2), Q3 = mul2(q3, q3);
   const float2 P23 = mul2(Q2, Q3), P13 = mul2(Q1, Q3), P12 = mul2(Q1, Q2);
   const float2 num = fma2(f2(1.5f), mul2(P12, sub2(tb, tc)), mul2(P23, sub2(ta, tb)));
-  // (scaled as in weno5_face2 the velocity arrays take 240 us at 256^3 for 227,
-  // and the error against FP64 is the same to 0.2 %)
   const float2 den = fma2(f2(3.0f), P12, fma2(f2(6.0f), P13, P23));
-  const float2 p2 = fma2(f2(3.0f), D3, fma2(f2(0.5f), e2, e3));
+  const float2 p2 = fma2(f2(0.5f), e2, e3);   // three times the candidate, less 3 D3
   float2 r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(den.x));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(den.y));
   r = fma2(r, fma2(mul2(f2(-1.0f), den), r, f2(1.0f)), r);
-  return mul2(fma2(num, r, p2), f2(inv * (1.0f / 3.0f)));
+  // D3 takes the exact 1/dx: the rounding error of a factor 1/(3 dx) on the
+  // whole is the same one in every derivative of an axis (mean error against
+  // FP64 at |phi| < 5 dx, 120 steps of velocity arrays at 160x144x130: 9.5e-9
+  // by that factor, 5.4e-9 so; the stage at 256^3 227.5 and 223.4 us)
+  return fma2(f2(inv), D3, mul2(fma2(num, r, p2), f2(inv * (1.0f / 3.0f))));
 }
 
 static __device__ __noinline__ float2 weno5_face_fp64(float u0, float u1, float u2,
