@@ -86,7 +86,8 @@ bool pairs_apply(const StageArgs& a) {
 // arithmetic; the face-shared kernel for the two-sided kinds, the one-sided
 // pair kernel for the upwind kinds) and pairs_apply; else one cell per
 // thread with the boundary values generated on the fly.  All cover TX x TY
-// x TZ cells per block, so the grid (and the per-block CFL partials) are
+// x p.tz cells per block (a narrow last column of tiles leaves blocks without
+// work, which report no speed), so the grid (and the per-block CFL partials) are
 // the same.
 template <typename T, int KIND>
 void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStream_t st) {
