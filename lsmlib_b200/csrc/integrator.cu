@@ -23,11 +23,6 @@
 
 using namespace lsmgpu;
 
-// z-slabs of the host-array driver's copies (see lsmgpu_normal_tvdrk3_host)
-#ifndef LSMGPU_HOST_SLABS
-#define LSMGPU_HOST_SLABS 4
-#endif
-constexpr int kHostSlabs = LSMGPU_HOST_SLABS;
 // speed buffers of queued host-array calls: up to kMaxSpeedBufs, as many as
 // fit in 1 GiB (at least 2)
 constexpr int kMaxSpeedBufs = 8;
@@ -548,8 +543,7 @@ int lsmgpu_workspace_create(lsmgpu_workspace** out, const int gb[6],
   ws->npart = kAdvRedBlocks;
   FillBox whole;
   for (int d = 0; d < 3; d++) { whole.lo[d] = ws->gb.lo[d]; whole.hi[d] = ws->gb.hi(d); }
-  // every slab of a host-array call takes its own blocks
-  const int most = stage_blocks_max(whole) + kHostSlabs * kStageMaxSplit;
+  const int most = stage_blocks_max(whole, kHostSlabs);
   if (most > ws->npart) ws->npart = most;
   if (!(ws->phi1 = ws_alloc(ws->bytes, R)) || !(ws->phi2 = ws_alloc(ws->bytes, R)) ||
       !(ws->rhs = ws_alloc(ws->bytes, R)) ||
@@ -1013,11 +1007,8 @@ int lsmgpu_normal_tvdrk3_host(lsmgpu_workspace* ws, void* phi, const void* F,
   // fill-box slabs on stage-tile boundaries in z, and the ghost-box planes
   // each slab owns: [zb[s], zb[s+1]) with the ghost planes below the fill box
   // in the first and those above it in the last
-  const int ntz = (f.n(2) + kStageTZ - 1) / kStageTZ;
-  const int ns = ntz < kHostSlabs ? ntz : kHostSlabs;
   int zlo[kHostSlabs + 1];
-  for (int q = 0; q <= ns; q++) zlo[q] = f.lo[2] + (int)((long)q * ntz / ns) * kStageTZ;
-  zlo[ns] = f.hi[2] + 1;
+  const int ns = stage_slabs(f, zlo);
   int zb[kHostSlabs + 1];
   for (int q = 0; q <= ns; q++) zb[q] = zlo[q];
   zb[0] = gb.lo[2];
@@ -1086,6 +1077,10 @@ int lsmgpu_normal_tvdrk3_host(lsmgpu_workspace* ws, void* phi, const void* F,
         b.fb = slab_fb(q);
         b.partials = ws->partials + off;
         off += stage_blocks(b.fb);
+        if (off > ws->npart) {
+          set_error(LSMGPU_ERR_INVALID_BOX, std::string(R) + ": slabs beyond the workspace");
+          return LSMGPU_ERR_INVALID_BOX;
+        }
         if (!cuda_ok(stage(kStageNormalRhs, ws->prec, b, st, ws), R)) return LSMGPU_ERR_CUDA;
       }
       nblk = off;   // the slabs' own blocks

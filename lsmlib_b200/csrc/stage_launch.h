@@ -81,10 +81,26 @@ inline int stage_tz(const FillBox& fb) {
   return best;
 }
 inline int stage_blocks(const FillBox& fb) { return stage_blocks(fb, stage_tz(fb)); }
-// the most blocks of any fill box inside `whole`
-inline int stage_blocks_max(const FillBox& whole) {
-  const int b = stage_blocks(whole, kStageMaxTZ);
-  return b > kStageMaxSplit ? b : kStageMaxSplit;
+// The z slabs of a host-array call (lsmgpu_normal_tvdrk3_host): slab q holds
+// planes [zlo[q], zlo[q + 1]) of the fill box, cut at multiples of kStageTZ.
+// Returns their number.
+constexpr int kHostSlabs = 4;
+inline int stage_slabs(const FillBox& fb, int zlo[kHostSlabs + 1]) {
+  const int layers = (fb.n(2) + kStageTZ - 1) / kStageTZ;
+  const int ns = layers < kHostSlabs ? layers : kHostSlabs;
+  for (int q = 0; q < ns; q++) zlo[q] = fb.lo[2] + (int)((long)q * layers / ns) * kStageTZ;
+  zlo[ns] = fb.hi[2] + 1;
+  return ns;
+}
+
+// At least the blocks of any fill box inside `whole`, taken as one or cut
+// along z into up to `slabs` boxes with blocks of their own.  A box of n
+// planes has at most kStageMaxSplit blocks or ceil(n / kStageMaxTZ) a column
+// of tiles, and each cut adds up to one layer of tiles to the sum of the latter.
+inline int stage_blocks_max(const FillBox& whole, int slabs = 1) {
+  FillBox w = whole;
+  w.hi[2] += (slabs - 1) * (kStageMaxTZ - 1);
+  return stage_blocks(w, kStageMaxTZ) + slabs * kStageMaxSplit;
 }
 
 // kind: StageKind; prec: 8 (FP64) or 4 (FP32)

@@ -1,0 +1,71 @@
+"""The host rules of the stage kernels' tiling, compiled from the header that the
+library uses: the buffer of per-block CFL maxima holds every launch's blocks."""
+import subprocess
+
+import pytest
+
+from lsmlib_b200 import build
+
+PROGRAM = r"""
+#include <cstdio>
+#include "stage_launch.h"
+using namespace lsmgpu;
+
+static FillBox box(int nx, int ny, int nz, int ghost) {
+  FillBox f;
+  const int n[3] = {nx, ny, nz};
+  for (int d = 0; d < 3; d++) {
+    f.lo[d] = -ghost;
+    f.hi[d] = n[d] - 1 + ghost;
+  }
+  return f;
+}
+
+int main() {
+  const int wide[] = {1,    8,    31,   33,   64,   129,  257,  512,  1023, 1448, 1536,
+                      2000, 2056, 2305, 2560, 3000, 4096, 8192, 20000};
+  long bad = 0;
+  for (int nx : wide)
+    for (int ny : wide)
+      for (int nz = 1; nz <= 400; nz++) {
+        const FillBox f = box(nx, ny, nz, 0);
+        const int room = stage_blocks_max(box(nx, ny, nz, 3), kHostSlabs);
+        int zlo[kHostSlabs + 1];
+        const int ns = stage_slabs(f, zlo);
+        long sum = 0;
+        bool cover = ns >= 1 && ns <= kHostSlabs && zlo[0] == 0 && zlo[ns] == nz;
+        for (int q = 0; q < ns; q++) {
+          FillBox s = f;
+          s.lo[2] = zlo[q];
+          s.hi[2] = zlo[q + 1] - 1;
+          cover = cover && s.n(2) >= 1;
+          sum += stage_blocks(s);
+        }
+        if (!cover || sum > room || stage_blocks(f) > room) {
+          if (bad++ < 5)
+            std::printf("%dx%dx%d: %d slabs, %ld blocks in all, %d whole, room for %d\n", nx, ny,
+                        nz, ns, sum, stage_blocks(f), room);
+        }
+      }
+  return bad != 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    def go(program):
+        d = tmp_path_factory.mktemp("tiling")
+        src, exe = str(d / "t.cu"), str(d / "t")
+        with open(src, "w") as f:
+            f.write(program)
+        subprocess.run([build.NVCC] + build.ARCH + ["-std=c++17", "-O1", "-I", build.CSRC, "-I",
+                                                    build.INCLUDE, src, "-o", exe],
+                       check=True, capture_output=True)
+        return subprocess.run([exe], capture_output=True, text=True)
+    return go
+
+
+def test_partials_hold_every_slab(run):
+    r = run(PROGRAM)
+    assert r.returncode == 0, r.stdout
