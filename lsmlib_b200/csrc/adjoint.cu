@@ -201,7 +201,7 @@ k_adjoint_stage(AdjParams p) {
   const int tcol = (tx < 3) ? tx : tx + 6;
   const int trow = (ty < 3) ? ty : ty + 6;
   // the ghost cells of the state hold its boundary values
-  auto ld = [&](int a, int b, int c) -> double { return __ldg(p.phi + aix(p.gb, a, b, c)); };
+  auto ld = [&](int a, int b, int c) -> double { return p.phi[aix(p.gb, a, b, c)]; };
 
   // registers of the next plane (loaded while the current one is worked):
   // the new top of the z window or the own cell (halo threads), the strip
@@ -212,9 +212,9 @@ k_adjoint_stage(AdjParams p) {
     if (act) {
       nx_c = ld(i, j, k + 3);
       const long o = aix(p.gb, i, j, k);
-      nv0 = __ldg(p.vel[0] + o);
-      nv1 = __ldg(p.vel[1] + o);
-      nv2 = __ldg(p.vel[2] + o);
+      nv0 = p.vel[0][o];
+      nv1 = p.vel[1][o];
+      nv2 = p.vel[2][o];
       nsa = p.src_a[o];
       if (p.src_b) nsb = p.src_b[o];
     } else if (ctr_halo) {

@@ -149,20 +149,20 @@ __device__ __forceinline__ T fetch_bc(const Grid3<const T>& g,
   if (m & kBcPeriodic) {
     const int nx = p.dom.hi[0] - p.dom.lo[0] + 1, ny = p.dom.hi[1] - p.dom.lo[1] + 1,
               nz = p.dom.hi[2] - p.dom.lo[2] + 1;
-    if (i < p.dom.lo[0] && (m & (1u << 16))) return __ldg(g.ptr(i + nx, j, k));
-    if (i > p.dom.hi[0] && (m & (2u << 16))) return __ldg(g.ptr(i - nx, j, k));
-    if (j < p.dom.lo[1] && (m & (4u << 16))) return __ldg(g.ptr(i, j + ny, k));
-    if (j > p.dom.hi[1] && (m & (8u << 16))) return __ldg(g.ptr(i, j - ny, k));
-    if (k < p.dom.lo[2] && (m & (16u << 16))) return __ldg(g.ptr(i, j, k + nz));
-    if (k > p.dom.hi[2] && (m & (32u << 16))) return __ldg(g.ptr(i, j, k - nz));
+    if (i < p.dom.lo[0] && (m & (1u << 16))) return g(i + nx, j, k);
+    if (i > p.dom.hi[0] && (m & (2u << 16))) return g(i - nx, j, k);
+    if (j < p.dom.lo[1] && (m & (4u << 16))) return g(i, j + ny, k);
+    if (j > p.dom.hi[1] && (m & (8u << 16))) return g(i, j - ny, k);
+    if (k < p.dom.lo[2] && (m & (16u << 16))) return g(i, j, k + nz);
+    if (k > p.dom.hi[2] && (m & (32u << 16))) return g(i, j, k - nz);
   }
   if (m & kBcCopy) {
-    if (i < p.dom.lo[0] && (m & (1u << 8))) return __ldg(g.ptr(p.dom.lo[0], j, k));
-    if (i > p.dom.hi[0] && (m & (2u << 8))) return __ldg(g.ptr(p.dom.hi[0], j, k));
-    if (j < p.dom.lo[1] && (m & (4u << 8))) return __ldg(g.ptr(i, p.dom.lo[1], k));
-    if (j > p.dom.hi[1] && (m & (8u << 8))) return __ldg(g.ptr(i, p.dom.hi[1], k));
-    if (k < p.dom.lo[2] && (m & (16u << 8))) return __ldg(g.ptr(i, j, p.dom.lo[2]));
-    if (k > p.dom.hi[2] && (m & (32u << 8))) return __ldg(g.ptr(i, j, p.dom.hi[2]));
+    if (i < p.dom.lo[0] && (m & (1u << 8))) return g(p.dom.lo[0], j, k);
+    if (i > p.dom.hi[0] && (m & (2u << 8))) return g(p.dom.hi[0], j, k);
+    if (j < p.dom.lo[1] && (m & (4u << 8))) return g(i, p.dom.lo[1], k);
+    if (j > p.dom.hi[1] && (m & (8u << 8))) return g(i, p.dom.hi[1], k);
+    if (k < p.dom.lo[2] && (m & (16u << 8))) return g(i, j, p.dom.lo[2]);
+    if (k > p.dom.hi[2] && (m & (32u << 8))) return g(i, j, p.dom.hi[2]);
   }
   const T* e;
   long inward;
@@ -180,9 +180,9 @@ __device__ __forceinline__ T fetch_bc(const Grid3<const T>& g,
   } else if (k > p.dom.hi[2] && (p.bc_mask & 32u)) {
     e = g.ptr(i, j, p.dom.hi[2]); inward = -g.sz; dist = k - p.dom.hi[2];
   } else {
-    return __ldg(g.ptr(i, j, k));
+    return g(i, j, k);
   }
-  const T e0 = __ldg(e), e1 = __ldg(e + inward);
+  const T e0 = *e, e1 = e[inward];
   const T slope = e0 - e1;
   return e0 + slope * (T)dist;
 }
@@ -387,7 +387,7 @@ __device__ __forceinline__ double stage_tile(const StageParams<T>& p, int bx,
   const int trow = (ty < 3) ? ty : ty + 6;
 
   auto ld = [&](int a, int b, int c) -> T {
-    return need_bc ? fetch_bc(phi, p, a, b, c) : __ldg(phi.ptr(a, b, c));
+    return need_bc ? fetch_bc(phi, p, a, b, c) : phi(a, b, c);
   };
 
   // registers of the plane to be written next: the new top of the z window
@@ -427,7 +427,7 @@ __device__ __forceinline__ double stage_tile(const StageParams<T>& p, int bx,
       // point loads of this cell, issued before the stencil arithmetic
       T a0 = T(0), a1 = T(0), a2 = T(0), uc = T(0);
       if (KIND == kStageAdvect) {
-        a0 = __ldg(p.aux0 + o); a1 = __ldg(p.aux1 + o); a2 = __ldg(p.aux2 + o);
+        a0 = p.aux0[o]; a1 = p.aux1[o]; a2 = p.aux2[o];
       } else if (KIND == kStageDeformation) {
         const int nx = p.fb.hi[0] - p.fb.lo[0] + 1, ny = p.fb.hi[1] - p.fb.lo[1] + 1,
                   nz = p.fb.hi[2] - p.fb.lo[2] + 1;
@@ -435,17 +435,17 @@ __device__ __forceinline__ double stage_tile(const StageParams<T>& p, int bx,
         const double* ty_ = p.defo_tab + p.defo_off[1] + (j - p.fb.lo[1]);
         const double* tz_ = p.defo_tab + p.defo_off[2] + (k - p.fb.lo[2]);
         DeformSines s;
-        s.sx = __ldg(tx_); s.s2x = __ldg(tx_ + nx);
-        s.sy = __ldg(ty_); s.s2y = __ldg(ty_ + ny);
-        s.sz = __ldg(tz_); s.s2z = __ldg(tz_ + nz);
-        deformation_velocity(s, __ldg(p.g_dev), a0, a1, a2);
+        s.sx = *tx_; s.s2x = tx_[nx];
+        s.sy = *ty_; s.s2y = ty_[ny];
+        s.sz = *tz_; s.s2z = tz_[nz];
+        deformation_velocity(s, *p.g_dev, a0, a1, a2);
       } else if (KIND == kStageAdvectConst) {
         a0 = p.vel_const[0]; a1 = p.vel_const[1]; a2 = p.vel_const[2];
       } else if (KIND == kStageNormal || KIND == kStageNormalRhs ||
                  (KIND == kStageReinit && p.use_phi0 == 1)) {
-        a0 = __ldg(p.aux0 + o);
+        a0 = p.aux0[o];
       }
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = __ldg(p.phi_n + o);
+      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = p.phi_n[o];
       T wx[7], wy[7];
       if constexpr (STAGING == 0) {
 #pragma unroll
@@ -607,7 +607,7 @@ __device__ __forceinline__ double stage_tile_faces(const StageParams<T>& p, int 
   const bool col_start = ty == TY - 1 && i <= hi0;
 
   auto ld = [&](int a, int b, int c) -> T {
-    return need_bc ? fetch_bc(phi, p, a, b, c) : __ldg(phi.ptr(a, b, c));
+    return need_bc ? fetch_bc(phi, p, a, b, c) : phi(a, b, c);
   };
   T nx_c = T(0), nx_hx = T(0), nx_hy = T(0);
   auto prefetch = [&](int k) {
@@ -644,8 +644,8 @@ __device__ __forceinline__ double stage_tile_faces(const StageParams<T>& p, int 
     if (act) {
       if (KIND == kStageNormal || KIND == kStageNormalRhs ||
           (KIND == kStageReinit && p.use_phi0 == 1))
-        a0 = __ldg(p.aux0 + o);
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = __ldg(p.phi_n + o);
+        a0 = p.aux0[o];
+      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = p.phi_n[o];
       T u[6], ym_next;
 #pragma unroll
       for (int m = 0; m < 6; m++) u[m] = tile[buf][ty + 3][tx + 1 + m];
@@ -796,7 +796,7 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
   // address arithmetic of every load was a twentieth of the integer work
   const T* P0 = p.phi_s + base0;
   const int isy = (int)sy, isz = (int)sz;
-  auto ld = [&](int a, int b, int c) -> T { return __ldg(P0 + (a + isy * b + isz * c)); };
+  auto ld = [&](int a, int b, int c) -> T { return P0[a + isy * b + isz * c]; };
   // next plane's values: the window tops (active cells) or the own cells
   // (halo cells), and the strip cells
   T n0 = T(0), n1 = T(0), na = T(0), nb = T(0), ny0 = T(0), ny1 = T(0);
@@ -860,12 +860,12 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
     T yp0 = T(0), yp1 = T(0), zp0 = T(0), zp1 = T(0), znx0 = T(0), znx1 = T(0);
     constexpr bool kAux = KIND == kStageNormal || KIND == kStageNormalRhs;
     if (act0) {
-      if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a00 = __ldg(p.aux0 + o0);
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc0 = __ldg(p.phi_n + o0);
+      if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a00 = p.aux0[o0];
+      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc0 = p.phi_n[o0];
     }
     if (act1) {
-      if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a01 = __ldg(p.aux0 + o0 + 1);
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc1 = __ldg(p.phi_n + o0 + 1);
+      if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a01 = p.aux0[o0 + 1];
+      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc1 = p.phi_n[o0 + 1];
     }
     if (act0) {
       // x: tile columns c0+2 .. c0+8 hold phi(x-2 .. x+4) of cell x = i0
@@ -1016,7 +1016,7 @@ __device__ __forceinline__ void stage_tile_pairs_up(
 
   const T* P0 = p.phi_s + base0;
   const int isy = (int)sy, isz = (int)sz;
-  auto ld = [&](int a, int b, int c) -> T { return __ldg(P0 + (a + isy * b + isz * c)); };
+  auto ld = [&](int a, int b, int c) -> T { return P0[a + isy * b + isz * c]; };
   T n0 = T(0), n1 = T(0), na = T(0), nb = T(0), ny0 = T(0), ny1 = T(0);
   auto prefetch = [&](int k) {
     if (act0) n0 = ld(i0, j, k + 3);
@@ -1069,7 +1069,7 @@ __device__ __forceinline__ void stage_tile_pairs_up(
       if (c == 1 && !act1) break;
       const long o = o0 + c;
       if (KIND == kStageAdvect) {
-        a[c][0] = __ldg(p.aux0 + o); a[c][1] = __ldg(p.aux1 + o); a[c][2] = __ldg(p.aux2 + o);
+        a[c][0] = p.aux0[o]; a[c][1] = p.aux1[o]; a[c][2] = p.aux2[o];
       } else if (KIND == kStageDeformation) {
         const int nx = p.fb.hi[0] - p.fb.lo[0] + 1, ny = p.fb.hi[1] - p.fb.lo[1] + 1,
                   nz = p.fb.hi[2] - p.fb.lo[2] + 1;
@@ -1077,14 +1077,14 @@ __device__ __forceinline__ void stage_tile_pairs_up(
         const double* ty_ = p.defo_tab + p.defo_off[1] + (j - p.fb.lo[1]);
         const double* tz_ = p.defo_tab + p.defo_off[2] + (k - p.fb.lo[2]);
         DeformSines sn;
-        sn.sx = __ldg(tx_); sn.s2x = __ldg(tx_ + nx);
-        sn.sy = __ldg(ty_); sn.s2y = __ldg(ty_ + ny);
-        sn.sz = __ldg(tz_); sn.s2z = __ldg(tz_ + nz);
-        deformation_velocity(sn, __ldg(p.g_dev), a[c][0], a[c][1], a[c][2]);
+        sn.sx = *tx_; sn.s2x = tx_[nx];
+        sn.sy = *ty_; sn.s2y = ty_[ny];
+        sn.sz = *tz_; sn.s2z = tz_[nz];
+        deformation_velocity(sn, *p.g_dev, a[c][0], a[c][1], a[c][2]);
       } else {
         a[c][0] = p.vel_const[0]; a[c][1] = p.vel_const[1]; a[c][2] = p.vel_const[2];
       }
-      if (p.rk_kind != 1) uc[c] = __ldg(p.phi_n + o);
+      if (p.rk_kind != 1) uc[c] = p.phi_n[o];
     }
     // one axis at a time for both cells, so that only one axis's stencils
     // are live: x from tile columns c0 .. c0+9 (phi(x0+2t-4 .. x0+2t+5)),
