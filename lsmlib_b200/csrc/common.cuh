@@ -122,9 +122,10 @@ __device__ __forceinline__ float sr_float(double x, unsigned r) {
 // block calls it first (a grid that ended without waiting would let its
 // successor overtake the grid before it).  It also lets the next kernel of
 // the chain become resident.  No effect in a kernel launched normally.
-// Such a kernel loads its arrays by ordinary loads: __ldg (and __restrict__)
-// promise data that does not change while the kernel is resident, which here
-// it may, and a load of that kind could be moved above the wait.
+// A kernel launched with launch_after loads its arrays by ordinary loads:
+// __ldg (and __restrict__) promise data that does not change while the kernel
+// is resident, which here it may, and a load of that kind could be moved
+// above the wait.
 __device__ __forceinline__ void grid_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");

@@ -149,20 +149,20 @@ __device__ __forceinline__ T fetch_bc(const Grid3<const T>& g,
   if (m & kBcPeriodic) {
     const int nx = p.dom.hi[0] - p.dom.lo[0] + 1, ny = p.dom.hi[1] - p.dom.lo[1] + 1,
               nz = p.dom.hi[2] - p.dom.lo[2] + 1;
-    if (i < p.dom.lo[0] && (m & (1u << 16))) return g(i + nx, j, k);
-    if (i > p.dom.hi[0] && (m & (2u << 16))) return g(i - nx, j, k);
-    if (j < p.dom.lo[1] && (m & (4u << 16))) return g(i, j + ny, k);
-    if (j > p.dom.hi[1] && (m & (8u << 16))) return g(i, j - ny, k);
-    if (k < p.dom.lo[2] && (m & (16u << 16))) return g(i, j, k + nz);
-    if (k > p.dom.hi[2] && (m & (32u << 16))) return g(i, j, k - nz);
+    if (i < p.dom.lo[0] && (m & (1u << 16))) return __ldg(g.ptr(i + nx, j, k));
+    if (i > p.dom.hi[0] && (m & (2u << 16))) return __ldg(g.ptr(i - nx, j, k));
+    if (j < p.dom.lo[1] && (m & (4u << 16))) return __ldg(g.ptr(i, j + ny, k));
+    if (j > p.dom.hi[1] && (m & (8u << 16))) return __ldg(g.ptr(i, j - ny, k));
+    if (k < p.dom.lo[2] && (m & (16u << 16))) return __ldg(g.ptr(i, j, k + nz));
+    if (k > p.dom.hi[2] && (m & (32u << 16))) return __ldg(g.ptr(i, j, k - nz));
   }
   if (m & kBcCopy) {
-    if (i < p.dom.lo[0] && (m & (1u << 8))) return g(p.dom.lo[0], j, k);
-    if (i > p.dom.hi[0] && (m & (2u << 8))) return g(p.dom.hi[0], j, k);
-    if (j < p.dom.lo[1] && (m & (4u << 8))) return g(i, p.dom.lo[1], k);
-    if (j > p.dom.hi[1] && (m & (8u << 8))) return g(i, p.dom.hi[1], k);
-    if (k < p.dom.lo[2] && (m & (16u << 8))) return g(i, j, p.dom.lo[2]);
-    if (k > p.dom.hi[2] && (m & (32u << 8))) return g(i, j, p.dom.hi[2]);
+    if (i < p.dom.lo[0] && (m & (1u << 8))) return __ldg(g.ptr(p.dom.lo[0], j, k));
+    if (i > p.dom.hi[0] && (m & (2u << 8))) return __ldg(g.ptr(p.dom.hi[0], j, k));
+    if (j < p.dom.lo[1] && (m & (4u << 8))) return __ldg(g.ptr(i, p.dom.lo[1], k));
+    if (j > p.dom.hi[1] && (m & (8u << 8))) return __ldg(g.ptr(i, p.dom.hi[1], k));
+    if (k < p.dom.lo[2] && (m & (16u << 8))) return __ldg(g.ptr(i, j, p.dom.lo[2]));
+    if (k > p.dom.hi[2] && (m & (32u << 8))) return __ldg(g.ptr(i, j, p.dom.hi[2]));
   }
   const T* e;
   long inward;
@@ -180,9 +180,9 @@ __device__ __forceinline__ T fetch_bc(const Grid3<const T>& g,
   } else if (k > p.dom.hi[2] && (p.bc_mask & 32u)) {
     e = g.ptr(i, j, p.dom.hi[2]); inward = -g.sz; dist = k - p.dom.hi[2];
   } else {
-    return g(i, j, k);
+    return __ldg(g.ptr(i, j, k));
   }
-  const T e0 = *e, e1 = e[inward];
+  const T e0 = __ldg(e), e1 = __ldg(e + inward);
   const T slope = e0 - e1;
   return e0 + slope * (T)dist;
 }
@@ -387,7 +387,7 @@ __device__ __forceinline__ double stage_tile(const StageParams<T>& p, int bx,
   const int trow = (ty < 3) ? ty : ty + 6;
 
   auto ld = [&](int a, int b, int c) -> T {
-    return need_bc ? fetch_bc(phi, p, a, b, c) : phi(a, b, c);
+    return need_bc ? fetch_bc(phi, p, a, b, c) : __ldg(phi.ptr(a, b, c));
   };
 
   // registers of the plane to be written next: the new top of the z window
@@ -427,7 +427,7 @@ __device__ __forceinline__ double stage_tile(const StageParams<T>& p, int bx,
       // point loads of this cell, issued before the stencil arithmetic
       T a0 = T(0), a1 = T(0), a2 = T(0), uc = T(0);
       if (KIND == kStageAdvect) {
-        a0 = p.aux0[o]; a1 = p.aux1[o]; a2 = p.aux2[o];
+        a0 = __ldg(p.aux0 + o); a1 = __ldg(p.aux1 + o); a2 = __ldg(p.aux2 + o);
       } else if (KIND == kStageDeformation) {
         const int nx = p.fb.hi[0] - p.fb.lo[0] + 1, ny = p.fb.hi[1] - p.fb.lo[1] + 1,
                   nz = p.fb.hi[2] - p.fb.lo[2] + 1;
@@ -435,17 +435,17 @@ __device__ __forceinline__ double stage_tile(const StageParams<T>& p, int bx,
         const double* ty_ = p.defo_tab + p.defo_off[1] + (j - p.fb.lo[1]);
         const double* tz_ = p.defo_tab + p.defo_off[2] + (k - p.fb.lo[2]);
         DeformSines s;
-        s.sx = *tx_; s.s2x = tx_[nx];
-        s.sy = *ty_; s.s2y = ty_[ny];
-        s.sz = *tz_; s.s2z = tz_[nz];
-        deformation_velocity(s, *p.g_dev, a0, a1, a2);
+        s.sx = __ldg(tx_); s.s2x = __ldg(tx_ + nx);
+        s.sy = __ldg(ty_); s.s2y = __ldg(ty_ + ny);
+        s.sz = __ldg(tz_); s.s2z = __ldg(tz_ + nz);
+        deformation_velocity(s, __ldg(p.g_dev), a0, a1, a2);
       } else if (KIND == kStageAdvectConst) {
         a0 = p.vel_const[0]; a1 = p.vel_const[1]; a2 = p.vel_const[2];
       } else if (KIND == kStageNormal || KIND == kStageNormalRhs ||
                  (KIND == kStageReinit && p.use_phi0 == 1)) {
-        a0 = p.aux0[o];
+        a0 = __ldg(p.aux0 + o);
       }
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = p.phi_n[o];
+      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = p.phi_n[o]; 
       T wx[7], wy[7];
       if constexpr (STAGING == 0) {
 #pragma unroll
@@ -607,7 +607,7 @@ __device__ __forceinline__ double stage_tile_faces(const StageParams<T>& p, int 
   const bool col_start = ty == TY - 1 && i <= hi0;
 
   auto ld = [&](int a, int b, int c) -> T {
-    return need_bc ? fetch_bc(phi, p, a, b, c) : phi(a, b, c);
+    return need_bc ? fetch_bc(phi, p, a, b, c) : __ldg(phi.ptr(a, b, c));
   };
   T nx_c = T(0), nx_hx = T(0), nx_hy = T(0);
   auto prefetch = [&](int k) {
@@ -644,8 +644,8 @@ __device__ __forceinline__ double stage_tile_faces(const StageParams<T>& p, int 
     if (act) {
       if (KIND == kStageNormal || KIND == kStageNormalRhs ||
           (KIND == kStageReinit && p.use_phi0 == 1))
-        a0 = p.aux0[o];
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = p.phi_n[o];
+        a0 = __ldg(p.aux0 + o);
+      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc = p.phi_n[o]; 
       T u[6], ym_next;
 #pragma unroll
       for (int m = 0; m < 6; m++) u[m] = tile[buf][ty + 3][tx + 1 + m];

@@ -81,6 +81,19 @@ inline int stage_tz(const FillBox& fb) {
   return best;
 }
 inline int stage_blocks(const FillBox& fb) { return stage_blocks(fb, stage_tz(fb)); }
+// The same for the one-cell kernels (256 threads, 3 blocks per SM), where no
+// partials depend on it: from 3 waves of blocks on 13 or 16 planes, whichever
+// takes fewer planes in whole waves.  Stages with boundary values made on the
+// fly, velocity arrays, FP64 and FP32: 384x320x200 703 and 537 us with 16
+// planes, 716 and 547 with stage_tz, 700 and 527 so; 200^3 279 and 220, 282
+// and 226, 277 and 219; 190x180x170 208 and 167 with 16, 213 and 173 with 13.
+inline int one_cell_tz(const FillBox& fb) {
+  constexpr int kSlots = 3 * 148;
+  const int b13 = stage_blocks(fb, 13), b16 = stage_blocks(fb, 16);
+  if (b13 < 3 * kSlots) return stage_tz(fb);
+  return (b16 + kSlots - 1) / kSlots * 18 < (b13 + kSlots - 1) / kSlots * 15 ? 16 : 13;
+}
+
 // The z slabs of a host-array call (lsmgpu_normal_tvdrk3_host): slab q holds
 // planes [zlo[q], zlo[q + 1]) of the fill box, cut at multiples of kStageTZ.
 // Returns their number.
