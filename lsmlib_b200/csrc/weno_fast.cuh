@@ -101,8 +101,12 @@ __device__ __forceinline__ float mantissa_of(float x) {
 // at the end), eps is taken from max|D|, the S_k and eps are taken four
 // times over, everything is formed from the second differences e_m =
 // D_m+1 - D_m, and with w2 = 1 - w1 - w3 and numerator and weight sum scaled
-//   3 phi = 3 p2 + (P23 T1 + 3/2 P12 T2) / (P23 + 6 P13 + 3 P12),
-// P_xy = (q_x q_y)^2, T1 = ta - tb, T2 = tb - tc the third differences.
+//   phi = D3 + (e3 + e2/2 + (P23 T1 + 3/2 P12 T2) / (P23 + 6 P13 + 3 P12)) / 3,
+// P_xy = (q_x q_y)^2, T1 = ta - tb, T2 = tb - tc the third differences.  D3
+// takes the exact 1/dx: a rounded 1/(3 dx) on the whole is the same error in
+// every derivative of an axis (mean relative error at dx = 2/160, emulated:
+// FP64 -8.5e-17 by that factor, 0 so, RMS 1.07e-16 and 4.6e-17; FP32 4.5e-8,
+// 0, RMS 5.8e-8 and 2.4e-8).
 // 53 FP64 instructions against 60 with the indicators from D directly.  FP64
 // stages at 257^3 (fill box): velocity arrays 446 -> 379 us, deformation field
 // 390 -> 378.
@@ -123,8 +127,8 @@ __device__ __forceinline__ T weno5_side_fast(T D1, T D2, T D3, T D4, T D5, T inv
   const T P23 = Q2 * Q3, P13 = Q1 * Q3, P12 = Q1 * Q2;
   const T num = fmaT(T(1.5), P12 * (tb - tc), P23 * (ta - tb));
   const T den = fmaT(T(3), P12, fmaT(T(6), P13, P23));
-  const T p2 = fmaT(T(3), D3, fmaT(T(0.5), e2, e3));
-  return fmaT(num, rcp_nr(den), p2) * (inv * T(1.0 / 3.0));
+  const T p2 = fmaT(T(0.5), e2, e3);   // three times the candidate, less 3 D3
+  return fmaT(inv, D3, fmaT(num, rcp_nr(den), p2) * (inv * T(1.0 / 3.0)));
 }
 
 // Weights and combination of one side from its smoothness indicators,
