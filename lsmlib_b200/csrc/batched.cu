@@ -540,22 +540,26 @@ int lsmgpu_batch_grid(lsmgpu_batch* b, int g, long long* offset, int gb[6]) {
   return LSMGPU_SUCCESS;
 }
 
-// copy the whole packed phi buffer from/to the host (grid g at its offset)
-int lsmgpu_batch_upload(lsmgpu_batch* b, const void* host) {
-  if (!batch_ok(b, "lsmgpu_batch_upload")) return LSMGPU_ERR_NULL_POINTER;
-  return cuda_ok(copy_to_device(b->phi, host, (size_t)b->total * b->prec, b->stream),
-                 "lsmgpu_batch_upload") &&
-                 cuda_ok(cudaStreamSynchronize(b->stream), "lsmgpu_batch_upload")
+// copy the whole packed phi buffer from/to the host (grid g at its offset):
+// behind the batch's own work and, as a cudaMemcpy, behind that of the legacy
+// default stream (which may still write or read the host buffer if it is
+// pinned; the batch's stream does not wait for it), complete on return
+static int batch_copy(lsmgpu_batch* b, void* host, bool to_host, const char* R) {
+  if (!batch_ok(b, R)) return LSMGPU_ERR_NULL_POINTER;
+  const size_t bytes = (size_t)b->total * b->prec;
+  return cuda_ok(cudaStreamSynchronize(b->stream), R) &&
+                 cuda_ok(to_host ? copy_to_host(host, b->phi, bytes, cudaStreamLegacy)
+                                 : copy_to_device(b->phi, host, bytes, cudaStreamLegacy),
+                         R) &&
+                 cuda_ok(cudaStreamSynchronize(cudaStreamLegacy), R)
              ? LSMGPU_SUCCESS
              : LSMGPU_ERR_CUDA;
 }
+int lsmgpu_batch_upload(lsmgpu_batch* b, const void* host) {
+  return batch_copy(b, const_cast<void*>(host), false, "lsmgpu_batch_upload");
+}
 int lsmgpu_batch_download(lsmgpu_batch* b, void* host) {
-  if (!batch_ok(b, "lsmgpu_batch_download")) return LSMGPU_ERR_NULL_POINTER;
-  return cuda_ok(copy_to_host(host, b->phi, (size_t)b->total * b->prec, b->stream),
-                 "lsmgpu_batch_download") &&
-                 cuda_ok(cudaStreamSynchronize(b->stream), "lsmgpu_batch_download")
-             ? LSMGPU_SUCCESS
-             : LSMGPU_ERR_CUDA;
+  return batch_copy(b, host, true, "lsmgpu_batch_download");
 }
 long long lsmgpu_batch_total_elements(lsmgpu_batch* b) { return b ? b->total : 0; }
 long long lsmgpu_batch_cells(lsmgpu_batch* b) { return b ? b->cells : 0; }
