@@ -565,17 +565,20 @@ StageArgs fwd_args(lsmgpu_adjoint* h) {
   a.dx_sq = m * m;
   a.dt = h->dt;
   for (int d = 0; d < 3; d++) a.aux[d] = h->vel[d];
-  // every stage input is one of the problem's own buffers: its ghost cells
-  // take the boundary values (checkpoint 0 holds a copy of the caller's phi0)
-  a.ghosts_writable = 1;
   return a;
 }
 
+// One stage.  Every stage input is one of the problem's own buffers: its ghost
+// cells take the boundary values here (checkpoint 0 holds a copy of the
+// caller's phi0), whichever kernel the stage runs in, and the reverse sweep
+// reads them as stored.
 cudaError_t fwd_stage(lsmgpu_adjoint* h, double* out, const double* in,
                       const double* base, int rk, cudaStream_t st) {
   StageArgs a = fwd_args(h);
-  a.out = out;
   a.phi_s = in;
+  if (cudaError_t e = launch_ghosts(8, a, st)) return e;
+  a.bc_mask = 0u;
+  a.out = out;
   a.phi_n = base;
   a.rk_kind = rk;
   return launch_stage_fast(kStageAdvect, 8, a, st);

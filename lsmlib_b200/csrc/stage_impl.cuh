@@ -43,10 +43,6 @@ StageParams<T> to_params(const StageArgs& a) {
   return p;
 }
 
-#ifndef LSMGPU_STAGE_PAIRS
-#define LSMGPU_STAGE_PAIRS 1
-#endif
-
 // The boundary values of a.bc_mask can be stored in phi_s's ghost cells:
 // the caller allows it, and every axis with a boundary kind has at least 3
 // domain cells (so no ghost value depends on another ghost cell).
@@ -93,7 +89,7 @@ template <typename T, int KIND>
 void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStream_t st) {
   constexpr int TX = kStageTX, TY = kStageTY;
   static_assert(TX == kPairTX && TY == kPairTY, "one tiling for all stage kernels");
-  if constexpr (LSMGPU_STAGE_PAIRS && UseFaces<T, KIND, STAGE_FAST, TX>::value) {
+  if constexpr (UseFaces<T, KIND, STAGE_FAST, TX>::value) {
     if (pairs_apply(a)) {
       StageParams<T> q = p;
       if (a.bc_mask != 0u) {
@@ -110,7 +106,7 @@ void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStr
       return;
     }
   }
-  if constexpr (LSMGPU_STAGE_PAIRS && UsePairsUp<T, KIND, STAGE_FAST, TX>::value) {
+  if constexpr (UsePairsUp<T, KIND, STAGE_FAST, TX>::value) {
     if (pairs_apply(a)) {
       StageParams<T> q = p;
       if (a.bc_mask != 0u) {
