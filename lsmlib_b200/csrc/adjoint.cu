@@ -514,8 +514,8 @@ struct lsmgpu_adjoint {
   double* theta = nullptr;
   double* grad_theta = nullptr;
   double* target = nullptr;
-  double* phi0 = nullptr;       // the initial state as given, ghost cells included
-  double* phi = nullptr;        // final state
+  double* phi = nullptr;        // final state, with phi0's ghost cells
+  bool fields_new = false;      // phi0 set since the last forward run
   double* s1 = nullptr;         // stage buffers
   double* s2 = nullptr;
   std::vector<double*> ckpt;    // checkpoint states
@@ -710,10 +710,16 @@ bool loss_to_host(lsmgpu_adjoint* h, double* loss, cudaStream_t st, const char* 
 
 // forward run from phi0 (h->ckpt[0] holds its interior), each step writing
 // straight into the next checkpoint where there is one; the final state is
-// left in h->phi, whose ghost cells are phi0's
+// left in h->phi, whose ghost cells are phi0's: the stages write interiors, and
+// h->phi is no stage's input, so one copy before checkpoint 0 takes boundary
+// values is enough
 cudaError_t forward_run(lsmgpu_adjoint* h, cudaStream_t st) {
-  cudaError_t e = cudaMemcpyAsync(h->phi, h->phi0, h->bytes, cudaMemcpyDeviceToDevice, st);
-  if (e) return e;
+  cudaError_t e;
+  if (h->fields_new) {
+    if ((e = cudaMemcpyAsync(h->phi, h->ckpt[0], h->bytes, cudaMemcpyDeviceToDevice, st)))
+      return e;
+    h->fields_new = false;
+  }
   double* const work = h->lam2;   // scratch of the reverse sweep
   for (int s = 0; s < h->nsteps; s++) {
     const double* in = s % h->every == 0 ? h->ckpt[s / h->every] : work;
@@ -771,7 +777,6 @@ int lsmgpu_adjoint_create(lsmgpu_adjoint** out, const int n[3], const double dx[
   h->theta = dalloc(3 * m3 * sizeof(double), ok);
   h->grad_theta = dalloc(3 * m3 * sizeof(double), ok);
   h->target = dalloc(h->bytes, ok);
-  h->phi0 = dalloc(h->bytes, ok);
   h->phi = dalloc(h->bytes, ok);
   h->s1 = dalloc(h->bytes, ok);
   h->s2 = dalloc(h->bytes, ok);
@@ -802,7 +807,7 @@ int lsmgpu_adjoint_create(lsmgpu_adjoint** out, const int n[3], const double dx[
 int lsmgpu_adjoint_destroy(lsmgpu_adjoint* h) {
   if (!h) return LSMGPU_SUCCESS;
   double* ps[] = {h->vel[0], h->vel[1], h->vel[2], h->A[0], h->A[1], h->A[2],
-                  h->theta, h->grad_theta, h->target, h->phi0, h->phi, h->s1, h->s2,
+                  h->theta, h->grad_theta, h->target, h->phi, h->s1, h->s2,
                   h->lam, h->lam2, h->lam1, h->T, h->Tb, h->partials};
   for (double* p : ps)
     if (p) cudaFree(p);
@@ -886,11 +891,9 @@ int lsmgpu_adjoint_set_fields(lsmgpu_adjoint* h, const double* phi0,
     return LSMGPU_ERR_NULL_POINTER;
   }
   h->eps = eps;
+  h->fields_new = true;
   cudaStream_t st = cur_stream();
-  return cuda_ok(cudaMemcpyAsync(h->phi0, phi0, h->bytes, cudaMemcpyHostToDevice, st), R) &&
-                 cuda_ok(cudaMemcpyAsync(h->ckpt[0], h->phi0, h->bytes,
-                                         cudaMemcpyDeviceToDevice, st),
-                         R) &&
+  return cuda_ok(cudaMemcpyAsync(h->ckpt[0], phi0, h->bytes, cudaMemcpyHostToDevice, st), R) &&
                  cuda_ok(cudaMemcpyAsync(h->target, target, h->bytes,
                                          cudaMemcpyHostToDevice, st),
                          R) &&
