@@ -41,6 +41,9 @@ constexpr int kStageTX = 32, kStageTY = 8, kStageTZ = 16;
 constexpr int kStageMaxTZ = 11;         // the longest march otherwise
 constexpr int kStageMaxSplit = 4096;    // shorter marches: at most this many blocks
 
+// a grid's z extent ends at 65535 blocks: the shortest march that covers fb
+inline int least_tz(const FillBox& fb) { return (fb.n(2) - 1) / 65535 + 1; }
+
 inline int stage_blocks(const FillBox& fb, int tz) {
   const int gx = (fb.n(0) + kStageTX - 1) / kStageTX;
   const int gy = (fb.n(1) + kStageTY - 1) / kStageTY;
@@ -67,6 +70,7 @@ inline int stage_tz(const FillBox& fb) {
   const long tiles = (long)(fb.n(0) / kStageTX) * ((fb.n(1) + kStageTY - 1) / kStageTY) +
                      (left ? (fb.n(1) + ly - 1) / ly : 0);
   int best = kStageMaxTZ;
+  if (least_tz(fb) > best) return least_tz(fb);
   double best_cost = 0.0;
   for (int tz = kStageMaxTZ; tz >= 1; tz--) {
     if (stage_blocks(fb, tz) > kStageMaxSplit) break;
@@ -91,7 +95,8 @@ inline int one_cell_tz(const FillBox& fb) {
   constexpr int kSlots = 3 * 148;
   const int b13 = stage_blocks(fb, 13), b16 = stage_blocks(fb, 16);
   if (b13 < 3 * kSlots) return stage_tz(fb);
-  return (b16 + kSlots - 1) / kSlots * 18 < (b13 + kSlots - 1) / kSlots * 15 ? 16 : 13;
+  const int tz = (b16 + kSlots - 1) / kSlots * 18 < (b13 + kSlots - 1) / kSlots * 15 ? 16 : 13;
+  return tz > least_tz(fb) ? tz : least_tz(fb);
 }
 
 // The z slabs of a host-array call (lsmgpu_normal_tvdrk3_host): slab q holds

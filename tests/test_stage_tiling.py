@@ -1,5 +1,6 @@
 """The host rules of the stage kernels' tiling, compiled from the header that the
-library uses: the buffer of per-block CFL maxima holds every launch's blocks."""
+library uses: the buffer of per-block CFL maxima holds every launch's blocks, and
+a launch's grid holds every plane."""
 import subprocess
 
 import pytest
@@ -52,6 +53,38 @@ int main() {
 """
 
 
+# grid extents of fill boxes with many planes (1,048,560 is what 16 planes a block
+# reach) and what a block marches
+TALL = r"""
+#include <cstdio>
+#include "stage_launch.h"
+using namespace lsmgpu;
+
+int main() {
+  long bad = 0;
+  const int planes[] = {1,      720884,  720885,  720886,  851955,   851956,
+                        900001, 1048559, 1048560, 1048561, 16000000, 2000000000};
+  for (int nx : {1, 8, 33, 64, 300})
+    for (int nz : planes) {
+      FillBox f;
+      const int n[3] = {nx, 1 + nx % 7, nz};
+      for (int d = 0; d < 3; d++) {
+        f.lo[d] = 0;
+        f.hi[d] = n[d] - 1;
+      }
+      for (int tz : {stage_tz(f), one_cell_tz(f)}) {
+        const long blocks = ((long)nz + tz - 1) / tz;
+        if (tz < 1 || blocks > 65535) {
+          bad++;
+          std::printf("%d planes: %d a block, %ld blocks\n", nz, tz, blocks);
+        }
+      }
+    }
+  return bad != 0;
+}
+"""
+
+
 @pytest.fixture(scope="module")
 def run(tmp_path_factory):
     def go(program):
@@ -64,6 +97,11 @@ def run(tmp_path_factory):
                        check=True, capture_output=True)
         return subprocess.run([exe], capture_output=True, text=True)
     return go
+
+
+def test_tall_boxes_fit_a_grid(run):
+    r = run(TALL)
+    assert r.returncode == 0, r.stdout
 
 
 def test_partials_hold_every_slab(run):
