@@ -66,10 +66,6 @@ __device__ __forceinline__ bool tless(const Time3& x, const Time3& y) {
   return x.a < y.a || (x.a == y.a && (x.b < y.b || (x.b == y.b && x.c < y.c)));
 }
 
-__device__ __forceinline__ bool tequal(const Time3& x, const Time3& y) {
-  return x.a == y.a && x.b == y.b && x.c == y.c;
-}
-
 // point x (time tx, linear index ix) is accepted before point y: by time,
 // exact ties by index
 __device__ __forceinline__ bool kless(const Time3& tx, long ix, const Time3& ty, long iy) {
@@ -82,18 +78,19 @@ __device__ __noinline__ bool kless_tied(Time3 tx, long ix, Time3 ty, long iy) {
   return kless(tx, ix, ty, iy);
 }
 
-// loads of values that other SMs write during the march: from L2, since an
-// L1 line may predate the write
-__device__ __forceinline__ Time3 ldcg(const Time3* t) {
-  return Time3{__ldcg(&t->a), __ldcg(&t->b), __ldcg(&t->c)};
-}
-
 // What an evaluation reads of a point: its value and the first level of its
 // time, with kKeyFront for a front point and kKeyOutside outside the domain
 // (times are >= 0) -- one 16-byte load in place of the value, the time and
-// the status byte.
+// the status byte.  The time's other levels lie in an array of their own.
 constexpr double kKeyFront = -1.0, kKeyOutside = -2.0;
 __device__ __forceinline__ bool key_inside(double k) { return k > -1.5; }
+
+// The whole time of a free point.  (Values that other SMs write during the
+// march are loaded from L2, since an L1 line may predate the write.)
+__device__ __forceinline__ Time3 time_of(const double2* vk, const double2* tm, long o) {
+  const double2 bc = __ldcg(tm + o);
+  return Time3{__ldcg(vk + o).y, bc.x, bc.y};
+}
 
 // linear index of the k-th point (k = 1, 2) from o in slot q's direction
 __device__ __forceinline__ long nb_index(long o, const long s[3], int q, int k) {
@@ -126,7 +123,7 @@ struct ExtSet {
 // the axes of the source interpolated linearly to the nearer crossing (or
 // taken from one side where the extension mask is < 0), weights
 // 1/d_axis^2 (:524-660).
-__global__ void k_fmm_front(double* d, Time3* tm, unsigned char* st, const double* phi,
+__global__ void k_fmm_front(double* d, double2* tm, unsigned char* st, const double* phi,
                             const double* mask, int nx, int ny, int nz, double dx,
                             double dy, double dz, ExtSet X) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -136,7 +133,7 @@ __global__ void k_fmm_front(double* d, Time3* tm, unsigned char* st, const doubl
   const double h[3] = {dx, dy, dz};
   for (int k = blockIdx.z; k < nz; k += gridDim.z) {
     const long o = (long)i + (long)nx * ((long)j + (long)ny * k);
-    tm[o] = Time3{INFINITY, INFINITY, INFINITY};
+    tm[o] = make_double2(INFINITY, INFINITY);
     if (mask && mask[o] < 0) {
       st[o] = kOutside;
       d[o] = DBL_MAX;
@@ -222,11 +219,11 @@ struct Eik {
 // marking before it (:214-246): points with mask < 0 or speed < 1e-11 are
 // outside the domain and get LSMLIB_REAL_MAX; points with phi > -1e-11 are
 // the front, KNOWN with their own values; the others start unreached.
-__global__ void k_eik_front(double* d, Time3* tm, unsigned char* st, const double* phi0,
+__global__ void k_eik_front(double* d, double2* tm, unsigned char* st, const double* phi0,
                             const double* speed, const double* mask, long n) {
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < n;
        o += (long)gridDim.x * blockDim.x) {
-    tm[o] = Time3{INFINITY, INFINITY, INFINITY};
+    tm[o] = make_double2(INFINITY, INFINITY);
     if ((mask && mask[o] < 0) || speed[o] < kZeroTol) {
       st[o] = kOutside;
       d[o] = DBL_MAX;
@@ -368,8 +365,9 @@ constexpr double kDeltaCells = 2.0, kDeltaCellsSmall = 6.0;
 // solver the point's input.  Neighbours off the grid
 // are left out, as the reference's bounds checks do.
 template <int ORDER, bool EIK>
-__device__ __noinline__ bool fmm_point(const double2* vk, const Time3* tm, long o, int c0, int c1, int c2, int nx, int ny, int nz,
-                                       double i2x, double i2y, double i2z, Eik E, Update* U) {
+__device__ __noinline__ bool fmm_point(const double2* vk, const double2* tm, long o, int c0,
+                                       int c1, int c2, int nx, int ny, int nz, double i2x,
+                                       double i2y, double i2z, Eik E, Update* U) {
   const int c[3] = {c0, c1, c2}, n[3] = {nx, ny, nz};
   const long s[3] = {1L, (long)nx, (long)nx * ny};
   const double i2[3] = {i2x, i2y, i2z};
@@ -387,14 +385,16 @@ __device__ __noinline__ bool fmm_point(const double2* vk, const Time3* tm, long 
     const double2 p1 = __ldcg(vk + o1);
     s1[q] = p1.y;
     nb.v1[q] = p1.x;
-    nb.t1[q] = ldcg(tm + o1);
+    const double2 bc1 = __ldcg(tm + o1);
+    nb.t1[q] = Time3{p1.y, bc1.x, bc1.y};
     if (ORDER == 2) {
       in2[q] = in1[q] && c[dir] + 2 * sg >= 0 && c[dir] + 2 * sg < n[dir];
       const long o2 = in2[q] ? o + 2 * sg * s[dir] : o;
       const double2 p2 = __ldcg(vk + o2);
       s2[q] = p2.y;
       nb.v2[q] = p2.x;
-      nb.t2[q] = ldcg(tm + o2);
+      const double2 bc2 = __ldcg(tm + o2);
+      nb.t2[q] = Time3{p2.y, bc2.x, bc2.y};
     }
   }
   nb.has1 = nb.front1 = nb.has2 = nb.front2 = 0;
@@ -530,7 +530,7 @@ __device__ __noinline__ bool fmm_point(const double2* vk, const Time3* tm, long 
 // behind).  The arithmetic of the coefficients and of the root is fmm_coeffs'
 // and fmm_root's.
 template <int ORDER, bool EIK>
-__device__ __forceinline__ int fmm_point_fast(const double2* vk, const Time3* tm, long o,
+__device__ __forceinline__ int fmm_point_fast(const double2* vk, const double2* tm, long o,
                                               const int c[3], const int n[3], const long s[3],
                                               const double i2[3], const Eik& E, Update& U,
                                               unsigned& readers) {
@@ -604,7 +604,7 @@ __device__ __forceinline__ int fmm_point_fast(const double2* vk, const Time3* tm
           for (int q = 0; q < 6; q++)
             if (tie >> q & 1) {
               const long iq = nb_index(o, s, q, 2);
-              if (kless_tied(ldcg(tm + iq), iq, ldcg(tm + it), it)) now |= 1u << q;
+              if (kless_tied(time_of(vk, tm, iq), iq, time_of(vk, tm, it), it)) now |= 1u << q;
             }
         }
       }
@@ -674,7 +674,7 @@ __device__ __forceinline__ int fmm_point_fast(const double2* vk, const Time3* tm
       for (unsigned m = eq; m; m &= m - 1) {
         const int q = __ffs(m) - 1;
         const long iq = nb_index(o, s, q, 1), ib = nb_index(o, s, best < 0 ? q : best, 1);
-        if (best < 0 || kless_tied(ldcg(tm + iq), iq, ldcg(tm + ib), ib)) best = q;
+        if (best < 0 || kless_tied(time_of(vk, tm, iq), iq, time_of(vk, tm, ib), ib)) best = q;
       }
       eq = 1u << best;
     }
@@ -765,8 +765,8 @@ struct Lists {
   int* pend_stamp;           // epoch + 1 that last queued a point
   double2* vk;               // per point: value and key (kKeyFront, kKeyOutside)
   double* new_d;             // per slot of the active list beyond each thread's
-  Time3* new_t;              //   first: the evaluated value, time and whether
-  unsigned char* new_f;      //   to store them
+  Time3* new_t;              //   first: the evaluated value (in the output
+  unsigned char* new_f;      //   array), time and whether to store them
 };
 
 // grid coordinates of point o (the entry points limit grids to 2^31 - 1
@@ -790,8 +790,8 @@ __device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
 
 // The points' pairs, and the first active list: the free points next to the
 // front.
-__global__ void k_fmm_seed(const double* d, const unsigned char* st, int nx, int ny, int nz, Lists L,
-                           Ctrl* ctrl) {
+__global__ void k_fmm_seed(const double* d, const unsigned char* st, int nx, int ny, int nz,
+                           Lists L, Ctrl* ctrl) {
   const long n = (long)nx * ny * nz;
   const long s[3] = {1L, (long)nx, (long)nx * ny};
   const int nn[3] = {nx, ny, nz};
@@ -962,9 +962,8 @@ __device__ __forceinline__ int2 reserve(int mine, int mine2, int* count, int* co
 // hardware one.
 template <int ORDER, bool EIK, bool CLUSTER>
 __global__ void __launch_bounds__(march_threads(ORDER, CLUSTER), 1)
-k_fmm_march(Time3* tm, int nx, int ny, int nz, double i2x, double i2y, double i2z, Lists L,
-            Ctrl* ctrl, ExtSet X, Eik E, double delta,
-            int max_passes) {
+k_fmm_march(double2* tm, int nx, int ny, int nz, double i2x, double i2y, double i2z, Lists L,
+            Ctrl* ctrl, ExtSet X, Eik E, double delta, int max_passes) {
   constexpr int kReaders = 6 * ORDER;
   __shared__ Room room;
   __shared__ unsigned long long s_min[2];
@@ -1024,7 +1023,7 @@ k_fmm_march(Time3* tm, int nx, int ny, int nz, double i2x, double i2y, double i2
         // only free points are ever queued; the value and time of the
         // point itself are loaded beside its stencil
         const double2 self = __ldcg(vk + o);
-        const double old = self.x, told_b = __ldcg(&tm[o].b);
+        const double old = self.x, told_b = __ldcg(&tm[o].x);
         int c[3];
         point_coords(o, nx, ny, c);
         Update U;
@@ -1054,7 +1053,7 @@ k_fmm_march(Time3* tm, int nx, int ny, int nz, double i2x, double i2y, double i2
         }
         // (the third level counts where the second does)
         const bool store = ext_changed || !(val == old && tv.a == self.y && tv.b == told_b &&
-                                            (tv.b == -1.0 || tv.c == __ldcg(&tm[o].c)));
+                                            (tv.b == -1.0 || tv.c == __ldcg(&tm[o].y)));
         if (base == 0) {
           f_first = store;
           o_first = (int)o;
@@ -1128,14 +1127,14 @@ k_fmm_march(Time3* tm, int nx, int ny, int nz, double i2x, double i2y, double i2
     if (!march_barrier<CLUSTER>(ctrl, gen, &s_ok)) return;
     if (f_first) {
       vk[o_first] = make_double2(d_first, t_first.a);
-      tm[o_first] = t_first;
+      tm[o_first] = make_double2(t_first.b, t_first.c);
     }
     for (int w = slot + total; w < count; w += total)
       if (L.new_f[w]) {
         const int o = __ldcg(cur + w);
         const Time3 t = L.new_t[w];
         vk[o] = make_double2(L.new_d[w], t.a);
-        tm[o] = t;
+        tm[o] = make_double2(t.b, t.c);
       }
     if (!march_barrier<CLUSTER>(ctrl, gen, &s_ok)) return;
     // thread 0 of each block: the threshold control, from the same words in
@@ -1178,22 +1177,21 @@ k_fmm_march(Time3* tm, int nx, int ny, int nz, double i2x, double i2y, double i2
   }
 }
 
-// The values of the free points; those no front reached take the reference's
-// default value -1 (distance
-// and extension fields), or the Eikonal solver's input
+// The values of all points (the march used the output array); free points no
+// front reached take the reference's default value -1 (distance and extension
+// fields), or the Eikonal solver's input
 __global__ void k_fmm_finish(double* d, const double2* vk, const unsigned char* st, long n,
                              ExtSet X, const double* phi0) {
   for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < n;
-       o += (long)gridDim.x * blockDim.x)
-    if (st[o] == kFree) {
-      const double v = vk[o].x;
-      if (fabs(v) <= DBL_MAX) {
-        d[o] = v;
-        continue;
-      }
-      d[o] = phi0 ? phi0[o] : -1.0;
-      for (int f = 0; f < X.nf; f++) X.ext[f][o] = -1.0;
+       o += (long)gridDim.x * blockDim.x) {
+    const double v = vk[o].x;
+    if (st[o] != kFree || fabs(v) <= DBL_MAX) {
+      d[o] = v;
+      continue;
     }
+    d[o] = phi0 ? phi0[o] : -1.0;
+    for (int f = 0; f < X.nf; f++) X.ext[f][o] = -1.0;
+  }
 }
 
 // One solve on device arrays: the distance function and up to kMaxFields
@@ -1210,21 +1208,21 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
   // few passes each
   const long max_passes = 4096 + 32L * (nx + ny + nz);
   unsigned char* status = nullptr;
-  Time3* tm = nullptr;
+  double2* tm = nullptr;
   // points of a typical list: two per point of the grid's largest cross-section
   const int longest = nx > ny ? (nx > nz ? nx : nz) : (ny > nz ? ny : nz);
   const long band = 2 * n / longest;
   Lists L{};
+  L.new_d = dd;   // the output, which k_fmm_finish writes
   Ctrl* ctrl = nullptr;
   const size_t un = (size_t)n;
   bool ok = cuda_ok(pool_alloc((void**)&status, un, st), R) &&
-            cuda_ok(pool_alloc((void**)&tm, un * sizeof(Time3), st), R) &&
+            cuda_ok(pool_alloc((void**)&tm, un * sizeof(double2), st), R) &&
             cuda_ok(pool_alloc((void**)&L.active, 2 * un * sizeof(int), st), R) &&
             cuda_ok(pool_alloc((void**)&L.pending, 2 * un * sizeof(int), st), R) &&
             cuda_ok(pool_alloc((void**)&L.stamp, un * sizeof(int), st), R) &&
             cuda_ok(pool_alloc((void**)&L.pend_stamp, un * sizeof(int), st), R) &&
             cuda_ok(pool_alloc((void**)&L.vk, un * sizeof(double2), st), R) &&
-            cuda_ok(pool_alloc((void**)&L.new_d, un * sizeof(double), st), R) &&
             cuda_ok(pool_alloc((void**)&L.new_t, un * sizeof(Time3), st), R) &&
             cuda_ok(pool_alloc((void**)&L.new_f, un, st), R) &&
             cuda_ok(pool_alloc((void**)&ctrl, sizeof(Ctrl), st), R);
@@ -1316,7 +1314,7 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     ok = cuda_ok(cudaGetLastError(), R);
   }
   for (void* q : {(void*)status, (void*)tm, (void*)L.active, (void*)L.pending,
-                  (void*)L.stamp, (void*)L.pend_stamp, (void*)L.vk, (void*)L.new_d, (void*)L.new_t,
+                  (void*)L.stamp, (void*)L.pend_stamp, (void*)L.vk, (void*)L.new_t,
                   (void*)L.new_f, (void*)ctrl})
     if (q) cudaFreeAsync(q, st);
   if (passes_out) *passes_out = h_ctrl.pass;
