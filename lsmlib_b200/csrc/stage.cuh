@@ -852,21 +852,28 @@ __device__ __forceinline__ double stage_tile_pairs(const StageParams<T>& p, int 
     if (has_a) tile[buf][ty + 3][cola] = na;
     if (has_b) tile[buf][ty + 3][colb] = nb;
     if (hy0 || hy1) *reinterpret_cast<T2*>(&tile[buf][trow][c0 + PX]) = T2{ny0, ny1};
-    __syncthreads();
-    if (k < ke) prefetch(k + 1);
     const long o0 = base0 + (i0 + isy * j + isz * k);
     T a00 = T(0), a01 = T(0), uc0 = T(0), uc1 = T(0);
+    constexpr bool kAux = KIND == kStageNormal || KIND == kStageNormalRhs;
+    auto point_loads = [&]() {
+      if (act0) {
+        if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a00 = p.aux0[o0];
+        if (KIND != kStageNormalRhs && p.rk_kind != 1) uc0 = p.phi_n[o0];
+      }
+      if (act1) {
+        if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a01 = p.aux0[o0 + 1];
+        if (KIND != kStageNormalRhs && p.rk_kind != 1) uc1 = p.phi_n[o0 + 1];
+      }
+    };
+    // (in FP64 before the barrier, which ordinary loads do not cross by
+    // themselves: normal speed at 256^3 341.8 -> 336.0 us, reinitialization
+    // 361.5 -> 360.8; FP32, with more warps, is slower so: 198 against 191)
+    if (sizeof(T) == 8) point_loads();
+    __syncthreads();
+    if (k < ke) prefetch(k + 1);
+    if (sizeof(T) == 4) point_loads();
     T xp0 = T(0), xp1 = T(0), xm1 = T(0), xnext = T(0);
     T yp0 = T(0), yp1 = T(0), zp0 = T(0), zp1 = T(0), znx0 = T(0), znx1 = T(0);
-    constexpr bool kAux = KIND == kStageNormal || KIND == kStageNormalRhs;
-    if (act0) {
-      if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a00 = p.aux0[o0];
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc0 = p.phi_n[o0];
-    }
-    if (act1) {
-      if (kAux || (KIND == kStageReinit && p.use_phi0 == 1)) a01 = p.aux0[o0 + 1];
-      if (KIND != kStageNormalRhs && p.rk_kind != 1) uc1 = p.phi_n[o0 + 1];
-    }
     if (act0) {
       // x: tile columns c0+2 .. c0+8 hold phi(x-2 .. x+4) of cell x = i0
       T u[7];
