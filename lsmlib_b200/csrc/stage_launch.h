@@ -51,17 +51,26 @@ inline int stage_blocks(const FillBox& fb, int tz) {
   return gx * gy * gz;
 }
 
-// Planes a block marches: the tz of the smallest estimated time.  A block
-// takes about tz + 2 planes (the window loads and the extra z faces cost
-// two), and a plane 2.1, 2.6, 3.2 or 3.5 us with 1 to 4 blocks on its SM
-// (more do not fit); blocks that follow one another without a common start
-// take 2.75 (measured on the FP64 reinitialization stage; the ratios hold for
-// the other kinds and FP32).  Small grids so get thin slabs that reach every
-// SM, larger ones slabs that end together: with 16 planes for every grid the
-// stage took 41.0 us at 33^3 (30 blocks), 43.0 at 65^3, 66.2 at
-// 130x98x132, now 12.4, 20.5 and 58.  Past 11 planes nothing is gained: 16
-// against 11 at 257^3 measured 407 and 404 us (reinitialization), 464 and 446
-// (velocity arrays).
+// Planes a block marches: the tz of the smallest estimated time of the FP64
+// pair kernels, four blocks per SM.  A block takes about tz + 2 planes (the
+// window loads and the extra z faces cost two), and a plane 2.1, 2.6, 3.2 or
+// 3.5 us with 1 to 4 blocks on its SM; blocks that follow one another without a
+// common start take 2.75 (fitted to the reinitialization stage).  Small grids
+// so get thin slabs that reach every SM, larger ones slabs that end together.
+// FP32 kernels hold five or six blocks per SM (kPairBlocks) and have no fit of
+// their own: the rule's choice takes up to 5 % more than the best tz from 160
+// cells an axis on, 10 % at 130, and up to 43 % more (still less than 16 planes
+// take, though) at 65 to 96.  Stages alone, launched back to back, in us
+// (reinitialization / velocity arrays):
+//                   FP64: 16 planes  best       rule     FP32: 16  best       rule
+//   33^3               34 / 29    5.7 / 4.9  5.7 / 4.8    23 / 17  4.3 / 3.3  4.3 / 3.4
+//   65^3               38 / 36     13 / 11    13 / 12     25 / 19  8.1 / 6.4   10 / 8.6
+//   96x80x88           38 / 36     20 / 18    20 / 19     25 / 19   13 / 9.0   15 / 13
+//   129x97x131         57 / 56     47 / 45    48 / 45     43 / 36   29 / 21    31 / 22
+//   161x145x131        94 / 96     78 / 77    79 / 78     59 / 39   48 / 36    49 / 36
+//   211x163x150       138 / 136   127 / 123  130 / 126    79 / 64   77 / 60    79 / 63
+//   257^3             387 / 379   382 / 372  384 / 373   233 / 179 230 / 176  232 / 178
+//   384x320x200       518 / 512   517 / 511  524 / 516   312 / 243 310 / 243  316 / 246
 inline int stage_tz(const FillBox& fb) {
   constexpr int kSms = 148, kSlots = 4 * kSms;
   constexpr double kSteady = 2.75, kPlane[5] = {0.0, 2.1, 2.6, 3.2, 3.5};
@@ -130,8 +139,8 @@ cudaError_t launch_stage_fast(int kind, int prec, const StageArgs& a,
 // the stencils of a.fb reach (at least 3 domain cells per axis).
 cudaError_t launch_ghosts(int prec, const StageArgs& a, cudaStream_t st);
 // One stage of kStageDeformation (velocity evaluated in the kernel, so both
-// precisions have it) in the FP64 band form, fast arithmetic: a32 and a64 name the same stage over the FP32
-// arrays and their FP64 copies; tile_fp64[tile] (tiles as in stage_blocks,
+// precisions have it) in the FP64 band form, fast arithmetic: a32 and a64 name
+// the same stage over the FP32 arrays and their FP64 copies; tile_fp64[tile] (tiles as in stage_blocks,
 // x fastest) = 1 computes the tile in FP64, 0 in FP32.  Both launches write
 // every output cell in both precisions.  cudaErrorNotSupported when the
 // two-cells-per-thread kernels do not apply (arrays of 2^31 or more cells,
