@@ -835,6 +835,29 @@ __host__ __device__ constexpr int march_threads(int order, bool cluster) {
 }
 constexpr int kClusterBlocks = 8;
 
+// Whether the march runs on one cluster: its barrier takes less than that of a
+// cooperative launch over the GPU, but its lists wait for the threads of 8 SMs.
+// The lists grow with the size of the fronts, some n^(1/2) on a plane and n^(2/3)
+// in space, and a point's evaluation takes about twice as long at second order,
+// a ninth longer with each field and a fifth less for the Eikonal solver.  Both
+// sides measured, in ms, cluster and GPU (six spheres, threshold steps of 6 cells):
+//   order 1:           362^2 6.6, 7.5    512^2 12.6, 12.2   1500^2  91, 48
+//   order 1, 8 fields: 181^2 3.9, 4.4    362^2 11.4, 10.4   1500^2 175, 67
+//   order 2:           181^2 3.8, 4.0    256^2  6.5, 6.3    1500^2 156, 58
+//   order 2, 8 fields: 128^2 3.7, 3.8    181^2  6.5, 6.2    1500^2 295, 97
+//   Eikonal:           362^2 6.1, 6.8    724^2 18.4, 16.5   1500^2  76, 42
+//   Eikonal, order 2:  256^2 5.6, 5.5    362^2  9.7, 8.5    1500^2 132, 52
+//   24^3: order 1 0.67, 0.72, order 2 1.5, 1.2; 32^3: 1.2, 1.0 and 2.8, 1.7
+// (The line was 1,536 cells on a plane's shorter side for every solve: 1500^2 had
+// become slower than with two kernels a pass, 137 ms at order 2.)
+bool march_on_cluster(const int* dims, int order, int fields, bool eikonal) {
+  const double n = (double)dims[0] * dims[1] * dims[2];
+  const bool flat = dims[0] == 1 || dims[1] == 1 || dims[2] == 1;
+  const double front = 2.0 * (flat ? sqrt(n) : cbrt(n * n));
+  const double line = (order == 1 ? 960.0 : 440.0) * (eikonal ? 1.25 : 1.0);
+  return front * (1.0 + fields / 9.0) <= line;
+}
+
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;   // +infinity
 
 // polls of a grid barrier before it gives up (seconds)
@@ -1258,9 +1281,9 @@ bool solve_device(double* dd, const double* dp, const double* dm, const ExtSet& 
     i2[q] = 1 / dx[q];
     i2[q] *= i2[q];
   }
-  // One cluster while the lists fit its threads, else one block per SM of a
+  // One cluster while its 8 SMs hold the lists, else one block per SM of a
   // cooperative launch; and the threshold's step
-  const bool cluster = band <= kClusterBlocks * 384;
+  const bool cluster = march_on_cluster(grid_dims, order, X.nf, E.speed != nullptr);
   const bool small = cluster || 4 * band <= (long)sms * march_threads(order, false);
   const double delta = (small ? kDeltaCellsSmall : kDeltaCells) * hmin;
   // (passes in whole batches of 32)

@@ -1,0 +1,76 @@
+"""The march on one cluster and over the GPU: the same bits on both sides of the
+line between them, for each solver and number of fields, and no grid that takes
+longer than a larger one for the side it was given."""
+import ctypes
+import time
+
+import numpy as np
+import pytest
+
+import oracle
+from lsmlib_b200 import gpu
+from test_fmm_golden import seeded_spheres
+from test_gpu_distance import (gpu_distance, gpu_eikonal, gpu_extension, lib,  # noqa: F401
+                               same_bits, seeded_eikonal)
+
+pytestmark = pytest.mark.gpu
+
+# planes of (2 m)(1 + fields / 9) <= 960 (order 1), 440 (order 2) take the cluster,
+# 1200 and 550 for the Eikonal solver; in space 2 m^2 <= the same
+DISTANCE = [((1, 480, 480), 1), ((1, 480, 481), 1), ((1, 220, 220), 2), ((1, 220, 221), 2),
+            ((21, 21, 21), 1), ((22, 22, 22), 1), ((14, 15, 15), 2), ((15, 15, 15), 2)]
+FIELDS = [((1, 432, 432), 1, 1), ((1, 432, 433), 1, 1), ((1, 254, 254), 1, 8), ((1, 254, 255), 1, 8),
+          ((1, 165, 165), 2, 3), ((1, 165, 166), 2, 3), ((1, 116, 116), 2, 8), ((1, 117, 117), 2, 8),
+          ((30, 31, 32), 2, 5)]
+EIKONAL = [((1, 600, 600), 1), ((1, 600, 601), 1), ((1, 275, 275), 2), ((1, 275, 276), 2)]
+
+
+@pytest.mark.parametrize("shape,order", DISTANCE)
+def test_distance(lib, shape, order):  # noqa: F811
+    phi, dx = seeded_spheres(shape, sum(shape))
+    got, _ = gpu_distance(lib, phi, order, dx)
+    assert same_bits(got, oracle.oracle_fmm(ordered=True)(phi, order, dx, None))
+
+
+@pytest.mark.parametrize("shape,order,fields", FIELDS)
+def test_extension(lib, shape, order, fields):  # noqa: F811
+    phi, dx = seeded_spheres(shape, sum(shape))
+    rng = np.random.default_rng(fields)
+    src = [rng.standard_normal(shape) for _ in range(fields)]
+    d, ext = gpu_extension(lib, phi, src, order, dx)
+    want_d, want_ext = oracle.oracle_extension(ordered=True)(phi, src, order, dx)
+    assert same_bits(d, want_d)
+    for a, b in zip(ext, want_ext):
+        assert same_bits(a, b)
+
+
+@pytest.mark.parametrize("shape,order", EIKONAL)
+def test_eikonal(lib, shape, order):  # noqa: F811
+    data, speed, dx = seeded_eikonal(shape, sum(shape))
+    got = gpu_eikonal(lib, data, speed, order, dx)
+    assert same_bits(got, oracle.oracle_eikonal(ordered=True)(data, speed, order, dx))
+
+
+def _seconds(lib, n, order, fields):  # noqa: F811
+    """The best of three solves on device arrays, after a first."""
+    shape = (n[2], n[1], n[0])
+    phi, dx = seeded_spheres(shape, 3, noise=0)
+    p = gpu.DeviceArray.from_host(phi.ravel())
+    out = [gpu.DeviceArray((phi.size,)) for _ in range(fields + 1)]
+    ptr = (ctypes.c_void_p * max(fields, 1))(*[q.ptr for q in out[1:]])
+    src = (ctypes.c_void_p * max(fields, 1))(*[p.ptr] * fields)
+    dims, h = (ctypes.c_int * 3)(*n), (ctypes.c_double * 3)(*dx)
+    took = []
+    for _ in range(4):
+        t = time.perf_counter()
+        gpu.check_rc(lib.lsmgpu_extension_fields3d(out[0].ptr, ptr, p.ptr, None, src, None,
+                                                   fields, order, dims, h, None), "solve")
+        gpu.check_rc(lib.lsmgpu_stream_synchronize(), "sync")
+        took.append(time.perf_counter() - t)
+    for q in [p] + out:
+        q.free()
+    return min(took[1:])
+
+
+def test_time_grows_with_the_plane(lib):  # noqa: F811
+    assert _seconds(lib, (1500, 1500, 1), 2, 0) < _seconds(lib, (2048, 2048, 1), 2, 0)
