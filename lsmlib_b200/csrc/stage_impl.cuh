@@ -129,7 +129,7 @@ void launch_kind(dim3 grid, const StageArgs& a, const StageParams<T>& p, cudaStr
   // 663 (the same in strict mode), 437 for 387 (FP32).
   StageParams<T> q = p;
   if (KIND != kStageNormalRhs && a.tz == 0) {
-    q.tz = one_cell_tz(a.fb);
+    q.tz = one_cell_tz(a.fb, (int)sizeof(T));
     grid.z = (a.fb.n(2) + q.tz - 1) / q.tz;
   }
   k_stage<T, KIND, STAGE_FAST, TX, TY><<<grid, dim3(TX, TY, 1), 0, st>>>(q);

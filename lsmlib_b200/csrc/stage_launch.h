@@ -94,18 +94,57 @@ inline int stage_tz(const FillBox& fb) {
   return best;
 }
 inline int stage_blocks(const FillBox& fb) { return stage_blocks(fb, stage_tz(fb)); }
-// The same for the one-cell kernels (256 threads, 3 blocks per SM), where no
-// partials depend on it: from 3 waves of blocks on 13 or 16 planes, whichever
-// takes fewer planes in whole waves.  Stages with boundary values made on the
-// fly, velocity arrays, FP64 and FP32: 384x320x200 703 and 537 us with 16
-// planes, 716 and 547 with stage_tz, 700 and 527 so; 200^3 279 and 220, 282
-// and 226, 277 and 219; 190x180x170 208 and 167 with 16, 213 and 173 with 13.
-inline int one_cell_tz(const FillBox& fb) {
-  constexpr int kSlots = 3 * 148;
+// The same for the one-cell kernels (256 threads, 3 blocks per SM: 444 at a
+// time), where no partials depend on it.  Thin slabs by stage_tz below 300 blocks
+// of 16 planes; then the march of 6 to 16 planes whose blocks end first
+// (one_cell_end); from 3 waves on 13 or 16, whichever takes fewer planes in whole
+// waves, 16 where both make as many layers.  Against the best march of 18 such
+// grids (boundary values made on the fly) the middle rule's choice takes 2 % more in FP64 and 3 % in FP32, stage_tz's 5 %,
+// 16 planes 14 % and 9 %.  In us (16 planes, stage_tz, this rule):
+//                strict, arrays   FP64, arrays     FP32, normal speed
+//   65^3           61, 37, 37      46, 28, 28       42, 27, 27
+//   40x1000x40    154, 161, 144   117, 113, 104    110, 114, 105
+//   200^3         404, 403, 403   279, 278, 278    240, 241, 242
+constexpr int kOneCellSlots = 3 * 148;
+
+// When the last block of a one-cell grid ends, in planes: the full layers' blocks
+// in whole waves, then the rest of them beside the blocks of the (thinner) last
+// layer.  A block starts in the time of half a plane in FP32 and of none in FP64;
+// a plane takes 0.4 and 0.85 of its time with one and two blocks on an SM.
+inline double one_cell_end(int columns, int nz, int tz, int prec) {
+  constexpr double kShare[4] = {0.4, 0.4, 0.85, 1.0};
+  const double start = prec == 8 ? 0.0 : 0.5;
+  const int layers = (nz + tz - 1) / tz, last = nz - (layers - 1) * tz;
+  const long full = (long)columns * (layers - 1);
+  const long rest = full % kOneCellSlots, free = kOneCellSlots - rest;
+  const long side = rest + columns < kOneCellSlots ? rest + columns : kOneCellSlots;
+  const double share = kShare[(side + 147) / 148];
+  const double by_full = rest ? (tz + start) * share : 0.0;
+  const double by_last = (double)((columns + free - 1) / free) * (last + start) * share;
+  return (double)(full / kOneCellSlots) * (tz + start) +
+         (by_full > by_last ? by_full : by_last);
+}
+
+inline int one_cell_tz(const FillBox& fb, int prec = 8) {
   const int b13 = stage_blocks(fb, 13), b16 = stage_blocks(fb, 16);
-  if (b13 < 3 * kSlots) return stage_tz(fb);
-  const int tz = (b16 + kSlots - 1) / kSlots * 18 < (b13 + kSlots - 1) / kSlots * 15 ? 16 : 13;
-  return tz > least_tz(fb) ? tz : least_tz(fb);
+  if (b16 < 300) return stage_tz(fb);
+  int best = 16;
+  if (b13 >= 3 * kOneCellSlots) {
+    const int w13 = (b13 + kOneCellSlots - 1) / kOneCellSlots,
+              w16 = (b16 + kOneCellSlots - 1) / kOneCellSlots;
+    if (b13 != b16 && w16 * 18 >= w13 * 15) best = 13;
+  } else {
+    const int columns = stage_blocks(fb, fb.n(2)), nz = fb.n(2);
+    double end = one_cell_end(columns, nz, best, prec);
+    for (int tz = 15; tz >= 6; tz--) {
+      const double e = one_cell_end(columns, nz, tz, prec);
+      if (e < end - 1e-9) {
+        best = tz;
+        end = e;
+      }
+    }
+  }
+  return best > least_tz(fb) ? best : least_tz(fb);
 }
 
 // The z slabs of a host-array call (lsmgpu_normal_tvdrk3_host): slab q holds
