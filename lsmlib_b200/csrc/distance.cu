@@ -997,8 +997,8 @@ __device__ __forceinline__ int2 reserve(int mine, int mine2, int* count, int* co
 // sectors: 35 us a pass at 68,000 points, 10.5 at 1,700).  9 to 14 us a pass
 // where the lists are short (half of it the evaluation, the rest the two
 // barriers and the queue), 31 at 68,000 points.
-// Lists that fit one cluster's threads run on 8 SMs, whose barrier is a
-// hardware one.
+// Short lists run on one cluster of 8 SMs, whose barrier is a hardware one
+// (march_on_cluster).
 // SOLVE: the distance function alone, with extension fields (whose values cost
 // registers that the others keep), or the Eikonal solver.
 enum { kSolveDistance, kSolveExtension, kSolveEikonal };
