@@ -94,13 +94,15 @@ inline int stage_tz(const FillBox& fb) {
   return best;
 }
 inline int stage_blocks(const FillBox& fb) { return stage_blocks(fb, stage_tz(fb)); }
+
 // The same for the one-cell kernels (256 threads, 3 blocks per SM: 444 at a
 // time), where no partials depend on it.  Thin slabs by stage_tz below 300 blocks
 // of 16 planes; then the march of 6 to 16 planes whose blocks end first
 // (one_cell_end); from 3 waves on 13 or 16, whichever takes fewer planes in whole
-// waves, 16 where both make as many layers.  Against the best march of 18 such
-// grids (boundary values made on the fly) the middle rule's choice takes 2 % more in FP64 and 3 % in FP32, stage_tz's 5 %,
-// 16 planes 14 % and 9 %.  In us (16 planes, stage_tz, this rule):
+// waves, 16 where both make as many layers.  Against the best march of 18 grids of
+// the middle kind (boundary values made on the fly) this rule's choice takes 2 %
+// more in FP64 and 3 % in FP32, stage_tz's 5 %, 16 planes 14 % and 9 %.  In us
+// (16 planes, stage_tz, this rule):
 //                strict, arrays   FP64, arrays     FP32, normal speed
 //   65^3           61, 37, 37      46, 28, 28       42, 27, 27
 //   40x1000x40    154, 161, 144   117, 113, 104    110, 114, 105
@@ -179,8 +181,8 @@ cudaError_t launch_stage_fast(int kind, int prec, const StageArgs& a,
 cudaError_t launch_ghosts(int prec, const StageArgs& a, cudaStream_t st);
 // One stage of kStageDeformation (velocity evaluated in the kernel, so both
 // precisions have it) in the FP64 band form, fast arithmetic: a32 and a64 name
-// the same stage over the FP32 arrays and their FP64 copies; tile_fp64[tile] (tiles as in stage_blocks,
-// x fastest) = 1 computes the tile in FP64, 0 in FP32.  Both launches write
+// the same stage over the FP32 arrays and their FP64 copies; tile_fp64[tile]
+// (tiles as in stage_blocks, x fastest) = 1 computes the tile in FP64, 0 in FP32.  Both launches write
 // every output cell in both precisions.  cudaErrorNotSupported when the
 // two-cells-per-thread kernels do not apply (arrays of 2^31 or more cells,
 // or boundary values that cannot be stored in the ghost cells).

@@ -19,9 +19,9 @@ pytestmark = pytest.mark.gpu
 # 1200 and 550 for the Eikonal solver; in space 2 m^2 <= the same
 DISTANCE = [((1, 480, 480), 1), ((1, 480, 481), 1), ((1, 220, 220), 2), ((1, 220, 221), 2),
             ((21, 21, 21), 1), ((22, 22, 22), 1), ((14, 15, 15), 2), ((15, 15, 15), 2)]
-FIELDS = [((1, 432, 432), 1, 1), ((1, 432, 433), 1, 1), ((1, 254, 254), 1, 8), ((1, 254, 255), 1, 8),
-          ((1, 165, 165), 2, 3), ((1, 165, 166), 2, 3), ((1, 116, 116), 2, 8), ((1, 117, 117), 2, 8),
-          ((30, 31, 32), 2, 5)]
+FIELDS = [((1, 432, 432), 1, 1), ((1, 432, 433), 1, 1), ((1, 254, 254), 1, 8),
+          ((1, 254, 255), 1, 8), ((1, 165, 165), 2, 3), ((1, 165, 166), 2, 3),
+          ((1, 116, 116), 2, 8), ((1, 117, 117), 2, 8), ((30, 31, 32), 2, 5)]
 EIKONAL = [((1, 600, 600), 1), ((1, 600, 601), 1), ((1, 275, 275), 2), ((1, 275, 276), 2)]
 
 
